@@ -1,4 +1,3 @@
-#include <atomic>
 // Persistent compressed all-reduce over peer-mapped NVLink memory (sm_100a).
 //
 // One cooperative launch per bucket performs the whole collective: rotation, scaling,
@@ -22,6 +21,9 @@
 #include <torch/extension.h>
 
 #include <cuda_bf16.h>
+
+#include <atomic>
+
 #include "fused_allreduce.cuh"
 
 namespace dq {
@@ -30,70 +32,69 @@ static constexpr int kBlock = 1024;  // codec block, elements
 
 // defined in fused_allreduce_b{2..8}.cu
 template <int BITS, typename T, int CODEC>
-void launch_one(const ARParams* host_params, const ARParams* dev_params, int nranks, int ctas, int threads,
-                cudaStream_t stream);
+void launch_one(const ARParams* params, int nranks, int ctas, int threads, cudaStream_t stream);
 
 template <typename T, int CODEC>
-static void launch_rht(int bits, const ARParams* hp, const ARParams* dp, int nranks, int ctas, int threads,
+static void launch_rht(int bits, const ARParams* hp, int nranks, int ctas, int threads,
                        cudaStream_t stream) {
   switch (bits) {
-    case 2: launch_one<2, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
-    case 3: launch_one<3, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
-    case 4: launch_one<4, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
-    case 5: launch_one<5, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
-    case 6: launch_one<6, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
-    case 7: launch_one<7, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
-    case 8: launch_one<8, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
+    case 2: launch_one<2, T, CODEC>(hp, nranks, ctas, threads, stream); break;
+    case 3: launch_one<3, T, CODEC>(hp, nranks, ctas, threads, stream); break;
+    case 4: launch_one<4, T, CODEC>(hp, nranks, ctas, threads, stream); break;
+    case 5: launch_one<5, T, CODEC>(hp, nranks, ctas, threads, stream); break;
+    case 6: launch_one<6, T, CODEC>(hp, nranks, ctas, threads, stream); break;
+    case 7: launch_one<7, T, CODEC>(hp, nranks, ctas, threads, stream); break;
+    case 8: launch_one<8, T, CODEC>(hp, nranks, ctas, threads, stream); break;
     default: TORCH_CHECK(false, "bits must be in 2..8, got ", bits);
   }
 }
 
 template <typename T, int CODEC>
-static void launch_sc(int bits, const ARParams* hp, const ARParams* dp, int nranks, int ctas, int threads,
+static void launch_sc(int bits, const ARParams* hp, int nranks, int ctas, int threads,
                       cudaStream_t stream) {
   switch (bits) {
-    case 2: launch_one<2, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
-    case 4: launch_one<4, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
-    case 8: launch_one<8, T, CODEC>(hp, dp, nranks, ctas, threads, stream); break;
+    case 2: launch_one<2, T, CODEC>(hp, nranks, ctas, threads, stream); break;
+    case 4: launch_one<4, T, CODEC>(hp, nranks, ctas, threads, stream); break;
+    case 8: launch_one<8, T, CODEC>(hp, nranks, ctas, threads, stream); break;
     default: TORCH_CHECK(false, "the superchunk codec has 2, 4 and 8 bit codes, got ", bits);
   }
 }
 
 template <typename T>
-static void launch_mx(int bits, const ARParams* hp, const ARParams* dp, int nranks, int ctas, int threads,
+static void launch_mx(int bits, const ARParams* hp, int nranks, int ctas, int threads,
                       cudaStream_t stream) {
   switch (bits) {
-    case 4: launch_one<4, T, kCodecMx>(hp, dp, nranks, ctas, threads, stream); break;
-    case 6: launch_one<6, T, kCodecMx>(hp, dp, nranks, ctas, threads, stream); break;
-    case 8: launch_one<8, T, kCodecMx>(hp, dp, nranks, ctas, threads, stream); break;
+    case 4: launch_one<4, T, kCodecMx>(hp, nranks, ctas, threads, stream); break;
+    case 6: launch_one<6, T, kCodecMx>(hp, nranks, ctas, threads, stream); break;
+    case 8: launch_one<8, T, kCodecMx>(hp, nranks, ctas, threads, stream); break;
     default: TORCH_CHECK(false, "the block-float codec has 4, 6 and 8 bit codes, got ", bits);
   }
 }
 
 template <typename T>
-static void launch_cast(int bits, const ARParams* hp, const ARParams* dp, int nranks, int ctas, int threads,
+static void launch_cast(int bits, const ARParams* hp, int nranks, int ctas, int threads,
                         cudaStream_t stream) {
   switch (bits) {
-    case 16: launch_one<16, T, kCodecCast>(hp, dp, nranks, ctas, threads, stream); break;
-    case 32: launch_one<32, T, kCodecCast>(hp, dp, nranks, ctas, threads, stream); break;
+    case 16: launch_one<16, T, kCodecCast>(hp, nranks, ctas, threads, stream); break;
+    case 32: launch_one<32, T, kCodecCast>(hp, nranks, ctas, threads, stream); break;
     default: TORCH_CHECK(false, "the identity wire carries bf16 (16) or fp32 (32) values, got ", bits);
   }
 }
 
 // `codec`: kCodecRht (SIMT rotation), kCodecRhtTc (tcgen05 rotation), kCodecScAee, kCodecScMee, kCodecMx
 template <typename T>
-static void launch_bits(int bits, const ARParams* hp, const ARParams* dp, int nranks, int ctas, int threads,
+static void launch_bits(int bits, const ARParams* hp, int nranks, int ctas, int threads,
                         cudaStream_t stream, int codec) {
   switch (codec) {
-    case kCodecRht: launch_rht<T, kCodecRht>(bits, hp, dp, nranks, ctas, threads, stream); break;
-    case kCodecRhtTc: launch_rht<T, kCodecRhtTc>(bits, hp, dp, nranks, ctas, threads, stream); break;
-    case kCodecScAee: launch_sc<T, kCodecScAee>(bits, hp, dp, nranks, ctas, threads, stream); break;
-    case kCodecScMee: launch_sc<T, kCodecScMee>(bits, hp, dp, nranks, ctas, threads, stream); break;
-    case kCodecMx: launch_mx<T>(bits, hp, dp, nranks, ctas, threads, stream); break;
-    case kCodecCast: launch_cast<T>(bits, hp, dp, nranks, ctas, threads, stream); break;
-    case kCodecScMixAee: launch_one<8, T, kCodecScMixAee>(hp, dp, nranks, ctas, threads, stream); break;
-    case kCodecScMixMee: launch_one<8, T, kCodecScMixMee>(hp, dp, nranks, ctas, threads, stream); break;
-    case kCodecRhtMix: launch_one<8, T, kCodecRhtMix>(hp, dp, nranks, ctas, threads, stream); break;
+    case kCodecRht: launch_rht<T, kCodecRht>(bits, hp, nranks, ctas, threads, stream); break;
+    case kCodecRhtTc: launch_rht<T, kCodecRhtTc>(bits, hp, nranks, ctas, threads, stream); break;
+    case kCodecScAee: launch_sc<T, kCodecScAee>(bits, hp, nranks, ctas, threads, stream); break;
+    case kCodecScMee: launch_sc<T, kCodecScMee>(bits, hp, nranks, ctas, threads, stream); break;
+    case kCodecMx: launch_mx<T>(bits, hp, nranks, ctas, threads, stream); break;
+    case kCodecCast: launch_cast<T>(bits, hp, nranks, ctas, threads, stream); break;
+    case kCodecScMixAee: launch_one<8, T, kCodecScMixAee>(hp, nranks, ctas, threads, stream); break;
+    case kCodecScMixMee: launch_one<8, T, kCodecScMixMee>(hp, nranks, ctas, threads, stream); break;
+    case kCodecRhtMix: launch_one<8, T, kCodecRhtMix>(hp, nranks, ctas, threads, stream); break;
     default: TORCH_CHECK(false, "unknown codec ", codec);
   }
 }
@@ -147,17 +148,14 @@ static void fill_sc(ARParams& p, int64_t codec, int64_t bits, double lattice_max
 static std::atomic<int> g_debug{0};
 void set_debug(bool on) { g_debug.store(on ? 1 : 0); }
 
-static void fill_common(ARParams& p, const at::Tensor& bucket, const at::Tensor& steps, int64_t rank, int64_t world,
+static void fill_common(ARParams& p, const at::Tensor& bucket, const int* steps, int64_t nsteps, int64_t rank, int64_t world,
                         int64_t blocks_per_shard, int64_t slot_stride, int64_t scales_off, int64_t flag_base,
                         int64_t epoch, int64_t seed, int64_t step, int64_t bucket_id, double post_scale,
                         int64_t timeout_ns, int64_t status_ptr, int64_t tail_ws_ptr, bool no_transmit) {
   TORCH_CHECK(bucket.is_cuda() && bucket.is_contiguous(), "bucket must be a contiguous CUDA tensor");
   TORCH_CHECK(bucket.scalar_type() == at::kFloat || bucket.scalar_type() == at::kBFloat16,
               "bucket must be float32 or bfloat16");
-  TORCH_CHECK(steps.device().is_cpu() && steps.scalar_type() == at::kInt && steps.dim() == 2 &&
-                  steps.size(1) == kStepInts && steps.is_contiguous(),
-              "steps must be a CPU int32 [nsteps, 8] tensor");
-  TORCH_CHECK(steps.size(0) <= kMaxSteps, "program too long");
+  TORCH_CHECK(nsteps <= kMaxSteps, "program too long");
   TORCH_CHECK(world >= 1 && world <= kMaxWorld && rank >= 0 && rank < world, "bad rank/world");
   p.bucket = bucket.data_ptr();
   p.n = bucket.numel();
@@ -166,7 +164,7 @@ static void fill_common(ARParams& p, const at::Tensor& bucket, const at::Tensor&
   TORCH_CHECK(p.blocks_per_shard * world >= p.nblocks, "shards do not cover the bucket");
   p.world = static_cast<int>(world);
   p.rank = static_cast<int>(rank);
-  p.nsteps = static_cast<int>(steps.size(0));
+  p.nsteps = static_cast<int>(nsteps);
   p.slot_stride = static_cast<unsigned long long>(slot_stride);
   p.scales_off = static_cast<unsigned long long>(scales_off);
   p.flag_base = static_cast<uint32_t>(flag_base);
@@ -181,9 +179,19 @@ static void fill_common(ARParams& p, const at::Tensor& bucket, const at::Tensor&
   p.tail_ws = reinterpret_cast<float*>(tail_ws_ptr);
   p.no_transmit = no_transmit ? 1 : 0;
   p.debug = g_debug.load();
-  const int* sp = steps.data_ptr<int>();
   for (int s = 0; s < p.nsteps; ++s)
-    for (int k = 0; k < kStepInts; ++k) p.steps[s][k] = sp[s * kStepInts + k];
+    for (int k = 0; k < kStepInts; ++k) {
+      const int v = steps[s * kStepInts + k];
+      TORCH_CHECK(v >= -32768 && v < 32768, "step ", s, ": field ", k, " does not fit 16 bits");
+      p.steps[s][k] = static_cast<short>(v);
+    }
+}
+
+// CPU int32 [.., nsteps, 8]
+static void check_steps(const at::Tensor& steps, int64_t dims) {
+  TORCH_CHECK(steps.device().is_cpu() && steps.scalar_type() == at::kInt && steps.dim() == dims &&
+                  steps.size(dims - 1) == kStepInts && steps.is_contiguous(),
+              "steps must be a contiguous CPU int32 tensor whose last dimension is 8");
 }
 
 static void check_layout(ARParams& p, int bits, int64_t mailbox_bytes, int64_t nslots, int64_t flag_words,
@@ -201,7 +209,7 @@ static void check_layout(ARParams& p, int bits, int64_t mailbox_bytes, int64_t n
               "mailbox too small for ", nslots, " slots");
   TORCH_CHECK(static_cast<long long>(p.flag_base) + nslots * ctas <= flag_words, "flag array too small");
   for (int s = 0; s < p.nsteps; ++s) {
-    const int* st = p.steps[s];
+    const short* st = p.steps[s];
     TORCH_CHECK(st[0] >= 0 && st[0] < p.world, "step ", s, ": bad shard");
     TORCH_CHECK(st[3] == 0 || (st[2] >= 0 && st[2] + st[3] <= nslots), "step ", s, ": bad receive slots");
     if (st[4] == kOutSend) TORCH_CHECK(st[5] >= 0 && st[5] < p.world && st[6] >= 0 && st[6] < nslots, "step ", s, ": bad send");
@@ -222,8 +230,9 @@ void fused_allreduce(at::Tensor bucket, at::Tensor steps, std::vector<int64_t> m
   TORCH_CHECK(static_cast<int64_t>(mail_ptrs.size()) == world && static_cast<int64_t>(flag_ptrs.size()) == world,
               "need one mailbox and one flag pointer per rank");
   TORCH_CHECK(threads % 32 == 0 && threads >= 32 && threads <= 512, "threads must be a multiple of 32, at most 512");
+  check_steps(steps, 2);
   ARParams p{};
-  fill_common(p, bucket, steps, rank, world, blocks_per_shard, slot_stride, scales_off, flag_base, epoch, seed, step,
+  fill_common(p, bucket, steps.data_ptr<int>(), steps.size(0), rank, world, blocks_per_shard, slot_stride, scales_off, flag_base, epoch, seed, step,
               bucket_id, post_scale, timeout_ns, status_ptr, tail_ws_ptr, no_transmit);
   fill_sc(p, codec, bits, sc_lattice_max, sc_c1, sc_c2, sc_lut, sc_plan);
   p.prefetch = prefetch ? 1 : 0;
@@ -234,9 +243,9 @@ void fused_allreduce(at::Tensor bucket, at::Tensor steps, std::vector<int64_t> m
   check_layout(p, static_cast<int>(bits), mailbox_bytes, nslots, flag_words, static_cast<int>(ctas));
   cudaStream_t stream = at::cuda::getCurrentCUDAStream();
   if (bucket.scalar_type() == at::kFloat)
-    launch_bits<float>(static_cast<int>(bits), &p, nullptr, 1, static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
+    launch_bits<float>(static_cast<int>(bits), &p, 1, static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
   else
-    launch_bits<__nv_bfloat16>(static_cast<int>(bits), &p, nullptr, 1, static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
+    launch_bits<__nv_bfloat16>(static_cast<int>(bits), &p, 1, static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
 }
 
 // All ranks of a collective in one launch on one GPU.  buckets[r], mailboxes[r] (uint8),
@@ -250,7 +259,8 @@ void fused_allreduce_local(std::vector<at::Tensor> buckets, at::Tensor steps, st
                      c10::optional<at::Tensor> sc_lut, c10::optional<at::Tensor> sc_plan, bool prefetch) {
   const int64_t world = static_cast<int64_t>(buckets.size());
   TORCH_CHECK(world >= 1 && world <= kMaxWorld, "1..8 ranks");
-  TORCH_CHECK(steps.dim() == 3 && steps.size(0) == world, "steps must be [world, nsteps, 8]");
+  check_steps(steps, 3);
+  TORCH_CHECK(steps.size(0) == world, "steps must be [world, nsteps, 8]");
   TORCH_CHECK(static_cast<int64_t>(mailboxes.size()) == world && static_cast<int64_t>(flags.size()) == world,
               "one mailbox and one flag array per rank");
   TORCH_CHECK(status.is_cuda() && status.scalar_type() == at::kInt && status.numel() >= 4, "status: 4 int32 words");
@@ -258,45 +268,34 @@ void fused_allreduce_local(std::vector<at::Tensor> buckets, at::Tensor steps, st
               "tail_ws: [world, 1024] float32");
   TORCH_CHECK(threads % 32 == 0 && threads >= 32 && threads <= 512, "threads must be a multiple of 32, at most 512");
   c10::cuda::CUDAGuard guard(buckets[0].device());
-  std::vector<ARParams> hp(world);
+  const int64_t nsteps = steps.size(1);
+  ARParamsSet set{};
   for (int64_t r = 0; r < world; ++r) {
     TORCH_CHECK(buckets[r].numel() == buckets[0].numel() && buckets[r].scalar_type() == buckets[0].scalar_type(),
                 "buckets must agree in size and dtype");
     TORCH_CHECK(mailboxes[r].is_cuda() && mailboxes[r].is_contiguous() && flags[r].is_cuda() &&
                     flags[r].scalar_type() == at::kInt,
                 "mailboxes / flags must be CUDA tensors");
-    hp[r] = ARParams{};
-    fill_common(hp[r], buckets[r], steps[r].contiguous(), r, world, blocks_per_shard, slot_stride, scales_off,
-                flag_base, epoch, seed, step, bucket_id, post_scale, timeout_ns,
+    ARParams& p = set.rank[r];
+    fill_common(p, buckets[r], steps.data_ptr<int>() + r * nsteps * kStepInts, nsteps, r, world, blocks_per_shard,
+                slot_stride, scales_off, flag_base, epoch, seed, step, bucket_id, post_scale, timeout_ns,
                 reinterpret_cast<int64_t>(status.data_ptr()),
                 reinterpret_cast<int64_t>(tail_ws.data_ptr<float>() + r * kBlock), no_transmit);
-    fill_sc(hp[r], codec, bits, sc_lattice_max, sc_c1, sc_c2, sc_lut, sc_plan);
-    hp[r].prefetch = prefetch ? 1 : 0;
+    fill_sc(p, codec, bits, sc_lattice_max, sc_c1, sc_c2, sc_lut, sc_plan);
+    p.prefetch = prefetch ? 1 : 0;
     for (int64_t q = 0; q < world; ++q) {
-      hp[r].mail[q] = static_cast<uint8_t*>(mailboxes[q].data_ptr());
-      hp[r].flags[q] = reinterpret_cast<uint32_t*>(flags[q].data_ptr());
+      set.rank[q].mail[r] = static_cast<uint8_t*>(mailboxes[r].data_ptr());
+      set.rank[q].flags[r] = reinterpret_cast<uint32_t*>(flags[r].data_ptr());
     }
-    check_layout(hp[r], static_cast<int>(bits), mailboxes[r].numel() * mailboxes[r].element_size(), nslots,
+    check_layout(p, static_cast<int>(bits), mailboxes[r].numel() * mailboxes[r].element_size(), nslots,
                  flags[r].numel(), static_cast<int>(ctas));
   }
+  // asynchronous: the parameters travel with the launch, nothing is waited for on the host
   cudaStream_t stream = at::cuda::getCurrentCUDAStream();
-  if (world == 1) {
-    if (buckets[0].scalar_type() == at::kFloat)
-      launch_bits<float>(static_cast<int>(bits), hp.data(), nullptr, 1, static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
-    else
-      launch_bits<__nv_bfloat16>(static_cast<int>(bits), hp.data(), nullptr, 1, static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
-    return;
-  }
-  at::Tensor dev = at::empty({static_cast<int64_t>(world * sizeof(ARParams))},
-                             at::TensorOptions().dtype(at::kByte).device(buckets[0].device()));
-  C10_CUDA_CHECK(cudaMemcpyAsync(dev.data_ptr(), hp.data(), world * sizeof(ARParams), cudaMemcpyHostToDevice, stream));
-  C10_CUDA_CHECK(cudaStreamSynchronize(stream));  // hp is pageable host memory
-  const ARParams* dp = reinterpret_cast<const ARParams*>(dev.data_ptr());
   if (buckets[0].scalar_type() == at::kFloat)
-    launch_bits<float>(static_cast<int>(bits), hp.data(), dp, static_cast<int>(world), static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
+    launch_bits<float>(static_cast<int>(bits), set.rank, static_cast<int>(world), static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
   else
-    launch_bits<__nv_bfloat16>(static_cast<int>(bits), hp.data(), dp, static_cast<int>(world), static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
-  C10_CUDA_CHECK(cudaStreamSynchronize(stream));  // keep `dev` alive until the kernel has read it
+    launch_bits<__nv_bfloat16>(static_cast<int>(bits), set.rank, static_cast<int>(world), static_cast<int>(ctas), static_cast<int>(threads), stream, static_cast<int>(codec));
 }
 
 }  // namespace dq

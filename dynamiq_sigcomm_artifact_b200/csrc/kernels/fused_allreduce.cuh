@@ -57,7 +57,13 @@ struct ARParams {
   int debug;                       // 1 (DQ_DEBUG=1 / debug=True): before a step touches a mailbox every CTA checks the
   int nslots;                      // step's slot indices against nslots, and the offset and length of every block of
   unsigned long long set_bytes;    // its range against the slot (plan-driven codecs: offsets come from device memory)
-  int steps[kMaxSteps][kStepInts];
+  short steps[kMaxSteps][kStepInts];  // 16 bits each (tags stay below 2^15): eight ranks' parameters fit one launch
+};
+
+// All ranks of a collective that runs in one launch on one GPU.  It is passed by value: 7 KB of kernel parameters cost
+// the launch nothing measurable, while a device copy of them needs an allocation, a transfer and a host wait per call.
+struct ARParamsSet {
+  ARParams rank[kMaxWorld];
 };
 
 }  // namespace dq

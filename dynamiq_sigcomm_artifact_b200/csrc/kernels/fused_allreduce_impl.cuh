@@ -44,7 +44,8 @@ __host__ __device__ constexpr size_t fused_smem_bytes(int threads, bool stage = 
   return nwarps * kBlock * 4 + (stage ? nwarps * kBlock * 4 : 0) + 2 * 4096 + 32 * 4 + nwarps * 8 + 64 + 128;
 }
 
-template <int BITS, typename T, int CODEC>
+// LOCAL: every rank runs in this launch, so flags and payloads never leave the GPU and device scope orders them.
+template <int BITS, typename T, int CODEC, bool LOCAL>
 __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
   constexpr bool MX = CODEC == kCodecMx;      // block-float codes (8 / 6 / 4 bit) with native conversions
   constexpr bool CAST = CODEC == kCodecCast;  // identity wire: bf16 (16) or fp32 (32) values
@@ -114,8 +115,7 @@ __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
     if (npend == 0) return;
     __syncthreads();  // every warp's payload stores of the pending steps precede their flags
     if (tid < npend) {
-      __threadfence_system();
-      st_release_sys(p.flags[pend[2 * tid]] + p.flag_base + static_cast<uint32_t>(pend[2 * tid + 1]) * G + cta, p.epoch);
+      publish_flag<LOCAL>(p.flags[pend[2 * tid]] + p.flag_base + static_cast<uint32_t>(pend[2 * tid + 1]) * G + cta, p.epoch);
     }
     npend = 0;
     __syncthreads();  // `pend` may be rewritten from here on
@@ -148,7 +148,7 @@ __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
       int bad_slot = 0;
       if (tid < nrecv) {
         const uint32_t* f = my_flags + p.flag_base + static_cast<uint32_t>(recv_slot + tid) * G + cta;
-        timed_out = !wait_flag(f, p.epoch, p.timeout_ns);
+        timed_out = !wait_flag<LOCAL>(f, p.epoch, p.timeout_ns);
         bad_slot = recv_slot + tid;
       }
       if (__syncthreads_or(timed_out)) {
@@ -444,8 +444,7 @@ __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
     } else if (out == kOutFinal) {
       __syncthreads();  // every warp's payload stores precede the flags
       if (tid < p.world && tid != p.rank) {
-        __threadfence_system();
-        st_release_sys(p.flags[tid] + p.flag_base + static_cast<uint32_t>(send_slot) * G + cta, p.epoch);
+        publish_flag<LOCAL>(p.flags[tid] + p.flag_base + static_cast<uint32_t>(send_slot) * G + cta, p.epoch);
       }
     }
   }
@@ -454,36 +453,34 @@ __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
   if (aborted && pf.s >= 0) mbar_wait(bar, pf_parity);  // let this warp's copy in flight land before leaving
 }
 
-template <int BITS, typename T, int CODEC>
+template <int BITS, typename T, int CODEC, bool LOCAL>
 __device__ __forceinline__ void fused_allreduce_body(const ARParams& p) {
   if constexpr (CODEC == kCodecRhtTc) rht_tc_body<BITS, T>(p);
-  else fused_simt_body<BITS, T, CODEC>(p);
+  else fused_simt_body<BITS, T, CODEC, LOCAL>(p);
 }
 
-// largest CTA of a codec's kernels (the tensor-core body trades a warpgroup for registers)
-template <int CODEC>
-constexpr int max_cta_threads() { return CODEC == kCodecRhtTc ? 512 : 512; }
+constexpr int kMaxCtaThreads = 512;
 
 template <int BITS, typename T, int CODEC>
-__global__ void __launch_bounds__(max_cta_threads<CODEC>(), 1) fused_allreduce_kernel(const __grid_constant__ ARParams p) {
-  fused_allreduce_body<BITS, T, CODEC>(p);
+__global__ void __launch_bounds__(kMaxCtaThreads, 1) fused_allreduce_kernel(const __grid_constant__ ARParams p) {
+  fused_allreduce_body<BITS, T, CODEC, false>(p);
 }
 
 // Several ranks in one launch on one GPU (blockIdx.y = rank): the single-GPU form of the
 // collective used by the standalone codec ops and by tests.  Cooperative, so that CTAs that
 // wait on one another are co-resident.
 template <int BITS, typename T, int CODEC>
-__global__ void __launch_bounds__(max_cta_threads<CODEC>(), 1) fused_allreduce_multi_kernel(const ARParams* __restrict__ plist) {
-  fused_allreduce_body<BITS, T, CODEC>(plist[blockIdx.y]);
+__global__ void __launch_bounds__(kMaxCtaThreads, 1) fused_allreduce_multi_kernel(const __grid_constant__ ARParamsSet set) {
+  fused_allreduce_body<BITS, T, CODEC, true>(set.rank[blockIdx.y]);
 }
 
+// `params`: one ARParams (nranks == 1) or the first entry of an ARParamsSet
 template <int BITS, typename T, int CODEC>
-void launch_one(const ARParams* host_params, const ARParams* dev_params, int nranks, int ctas, int threads,
-                cudaStream_t stream) {
+void launch_one(const ARParams* params, int nranks, int ctas, int threads, cudaStream_t stream) {
   constexpr bool TC = CODEC == kCodecRhtTc;
   TORCH_CHECK(!TC || (threads % 128 == 0 && threads >= 128 && threads <= 512),
               "the tensor-core rotation runs with 1 to 4 whole warpgroups (128, 256, 384 or 512 threads)");
-  const bool stage = host_params == nullptr || host_params->prefetch != 0;
+  const bool stage = params->prefetch != 0;
   const size_t smem = fused_smem_bytes<TC>(threads, stage);
   const void* fn = nranks == 1 ? reinterpret_cast<const void*>(&fused_allreduce_kernel<BITS, T, CODEC>)
                                : reinterpret_cast<const void*>(&fused_allreduce_multi_kernel<BITS, T, CODEC>);
@@ -508,47 +505,40 @@ void launch_one(const ARParams* host_params, const ARParams* dev_params, int nra
   }
   TORCH_CHECK(static_cast<long long>(ctas) * nranks <= c.capacity, "fused all-reduce: ", ctas, " CTAs x ", nranks,
               " ranks do not fit co-resident (capacity ", c.capacity, " CTAs of ", threads, " threads)");
-  dim3 grid(ctas, nranks), block(threads);
-  if (nranks == 1) {
-    void* args[] = {const_cast<ARParams*>(host_params)};
-    C10_CUDA_CHECK(cudaLaunchCooperativeKernel(fn, grid, block, args, smem, stream));
-  } else {
-    void* args[] = {&dev_params};
-    C10_CUDA_CHECK(cudaLaunchCooperativeKernel(fn, grid, block, args, smem, stream));
-  }
+  void* args[] = {const_cast<ARParams*>(params)};
+  C10_CUDA_CHECK(cudaLaunchCooperativeKernel(fn, dim3(ctas, nranks), dim3(threads), args, smem, stream));
 }
 
-
 #define DQ_INSTANTIATE_FUSED_ALLREDUCE(BITS)                                                                   \
-  template void launch_one<BITS, float, kCodecRht>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);           \
-  template void launch_one<BITS, __nv_bfloat16, kCodecRht>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);   \
-  template void launch_one<BITS, float, kCodecRhtTc>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);         \
-  template void launch_one<BITS, __nv_bfloat16, kCodecRhtTc>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);
+  template void launch_one<BITS, float, kCodecRht>(const ARParams*, int, int, int, cudaStream_t);           \
+  template void launch_one<BITS, __nv_bfloat16, kCodecRht>(const ARParams*, int, int, int, cudaStream_t);   \
+  template void launch_one<BITS, float, kCodecRhtTc>(const ARParams*, int, int, int, cudaStream_t);         \
+  template void launch_one<BITS, __nv_bfloat16, kCodecRhtTc>(const ARParams*, int, int, int, cudaStream_t);
 
 #define DQ_INSTANTIATE_FUSED_ALLREDUCE_CAST(BITS)                                                                       \
-  template void launch_one<BITS, float, kCodecCast>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);         \
-  template void launch_one<BITS, __nv_bfloat16, kCodecCast>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);
+  template void launch_one<BITS, float, kCodecCast>(const ARParams*, int, int, int, cudaStream_t);         \
+  template void launch_one<BITS, __nv_bfloat16, kCodecCast>(const ARParams*, int, int, int, cudaStream_t);
 
 #define DQ_INSTANTIATE_FUSED_ALLREDUCE_MX(BITS)                                                                         \
-  template void launch_one<BITS, float, kCodecMx>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);           \
-  template void launch_one<BITS, __nv_bfloat16, kCodecMx>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);
+  template void launch_one<BITS, float, kCodecMx>(const ARParams*, int, int, int, cudaStream_t);           \
+  template void launch_one<BITS, __nv_bfloat16, kCodecMx>(const ARParams*, int, int, int, cudaStream_t);
 
 #define DQ_INSTANTIATE_FUSED_ALLREDUCE_SC(BITS)                                                                         \
-  template void launch_one<BITS, float, kCodecScAee>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);         \
-  template void launch_one<BITS, __nv_bfloat16, kCodecScAee>(const ARParams*, const ARParams*, int, int, int, cudaStream_t); \
-  template void launch_one<BITS, float, kCodecScMee>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);         \
-  template void launch_one<BITS, __nv_bfloat16, kCodecScMee>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);
+  template void launch_one<BITS, float, kCodecScAee>(const ARParams*, int, int, int, cudaStream_t);         \
+  template void launch_one<BITS, __nv_bfloat16, kCodecScAee>(const ARParams*, int, int, int, cudaStream_t); \
+  template void launch_one<BITS, float, kCodecScMee>(const ARParams*, int, int, int, cudaStream_t);         \
+  template void launch_one<BITS, __nv_bfloat16, kCodecScMee>(const ARParams*, int, int, int, cudaStream_t);
 
 // rotation codec with a width per block: the BITS parameter is a placeholder (8, the widest block)
 #define DQ_INSTANTIATE_FUSED_ALLREDUCE_RHTMIX                                                                           \
-  template void launch_one<8, float, kCodecRhtMix>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);         \
-  template void launch_one<8, __nv_bfloat16, kCodecRhtMix>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);
+  template void launch_one<8, float, kCodecRhtMix>(const ARParams*, int, int, int, cudaStream_t);         \
+  template void launch_one<8, __nv_bfloat16, kCodecRhtMix>(const ARParams*, int, int, int, cudaStream_t);
 
 // mixed-width superchunk codec: the BITS parameter is a placeholder (8, the widest record)
 #define DQ_INSTANTIATE_FUSED_ALLREDUCE_SCMIX                                                                              \
-  template void launch_one<8, float, kCodecScMixAee>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);         \
-  template void launch_one<8, __nv_bfloat16, kCodecScMixAee>(const ARParams*, const ARParams*, int, int, int, cudaStream_t); \
-  template void launch_one<8, float, kCodecScMixMee>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);         \
-  template void launch_one<8, __nv_bfloat16, kCodecScMixMee>(const ARParams*, const ARParams*, int, int, int, cudaStream_t);
+  template void launch_one<8, float, kCodecScMixAee>(const ARParams*, int, int, int, cudaStream_t);         \
+  template void launch_one<8, __nv_bfloat16, kCodecScMixAee>(const ARParams*, int, int, int, cudaStream_t); \
+  template void launch_one<8, float, kCodecScMixMee>(const ARParams*, int, int, int, cudaStream_t);         \
+  template void launch_one<8, __nv_bfloat16, kCodecScMixMee>(const ARParams*, int, int, int, cudaStream_t);
 
 }  // namespace dq

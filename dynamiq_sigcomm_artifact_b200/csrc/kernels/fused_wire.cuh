@@ -26,13 +26,38 @@ __device__ __forceinline__ unsigned long long now_ns() {
 }
 __device__ __forceinline__ uint32_t ld_cg_u32(const uint32_t* p) { return __ldcg(p); }
 
+__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+template <bool LOCAL>
+__device__ __forceinline__ uint32_t read_flag(const uint32_t* flag) {
+  return LOCAL ? ld_acquire_gpu(flag) : ld_acquire_sys(flag);
+}
+
+// Publish what the CTA's warps stored before the last block barrier.
+template <bool LOCAL>
+__device__ __forceinline__ void publish_flag(uint32_t* flag, uint32_t epoch) {
+  if (LOCAL) {
+    st_release_gpu(flag, epoch);
+  } else {
+    __threadfence_system();
+    st_release_sys(flag, epoch);
+  }
+}
+
 // Wait until *flag reaches `epoch`; false when the budget ran out.
+template <bool LOCAL = false>
 __device__ __forceinline__ bool wait_flag(const uint32_t* flag, uint32_t epoch, unsigned long long budget_ns) {
-  if (static_cast<int32_t>(ld_acquire_sys(flag) - epoch) >= 0) return true;
+  if (static_cast<int32_t>(read_flag<LOCAL>(flag) - epoch) >= 0) return true;
   const unsigned long long t0 = now_ns();
   unsigned spins = 0;
   for (;;) {
-    if (static_cast<int32_t>(ld_acquire_sys(flag) - epoch) >= 0) return true;
+    if (static_cast<int32_t>(read_flag<LOCAL>(flag) - epoch) >= 0) return true;
     if ((++spins & 63u) == 0) {
       if (now_ns() - t0 > budget_ns) return false;
       __nanosleep(64);

@@ -15,6 +15,7 @@ Reference counterparts: the ring / butterfly callbacks and their per-tag send/re
 from __future__ import annotations
 
 import dataclasses
+import functools
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
@@ -71,19 +72,19 @@ class Layout:
     bits: int
     codec: str = "rht"
 
-    @property
+    @functools.cached_property
     def nblocks(self) -> int:
         return (self.numel + BLOCK - 1) // BLOCK
 
-    @property
+    @functools.cached_property
     def blocks_per_shard(self) -> int:
         return sch.shard_blocks(self.nblocks, self.world)
 
-    @property
+    @functools.cached_property
     def scales_off(self) -> int:
         return _align(self.blocks_per_shard * block_bytes(self.bits, self.codec), 16)
 
-    @property
+    @functools.cached_property
     def slot_stride(self) -> int:
         scales = 4 * self.blocks_per_shard if self.codec in RHT_CODECS else 0
         return _align(self.scales_off + scales, 256)
@@ -375,15 +376,40 @@ class LocalCluster:
         self.mail = [torch.zeros(self.mailbox_bytes, dtype=torch.uint8, device=self.device) for _ in range(world)]
         self.flags = [torch.zeros(self.nslots * ctas, dtype=torch.int32, device=self.device) for _ in range(world)]
         self.status = torch.zeros(4, dtype=torch.int32, device=self.device)
+        self._device_index = self.status.device.index
         self.tail_ws = torch.zeros(world, BLOCK, dtype=torch.float32, device=self.device)
         self.epoch = 0
+        self._programs: Dict[tuple, torch.Tensor] = {}
+        self._layouts: Dict[tuple, Layout] = {}
+        self._last_stream: Optional[torch.cuda.Stream] = None
+        self._last_stream_id: Optional[int] = None
+
+    def _join_streams(self) -> None:
+        """Mailboxes and flags are reused by every call: a call on another stream than the last one's waits for it."""
+        raw = torch._C._cuda_getCurrentRawStream(self._device_index)
+        if raw == self._last_stream_id:
+            return
+        stream = torch.cuda.current_stream(self.device)
+        if self._last_stream is not None:
+            stream.wait_stream(self._last_stream)
+        self._last_stream, self._last_stream_id = stream, raw
+
+    def _layout(self, numel: int, bits: int, codec: str) -> Layout:
+        key = (numel, bits, codec)
+        lay = self._layouts.get(key)
+        if lay is None:
+            if len(self._layouts) >= 64:
+                self._layouts.clear()
+            lay = self._layouts[key] = Layout(numel, self.world, bits, codec)
+        return lay
 
     def run(self, buckets: List[torch.Tensor], programs: torch.Tensor, bits: int, seed: int = 0, step: int = 0,
             bucket_id: int = 0, post_scale: Optional[float] = None, no_transmit: bool = False,
             preset_flags: bool = False, codec: Optional[str] = None, plan: Optional[torch.Tensor] = None) -> None:
         codec = codec or ("rht_tc" if self.tensor_rotation else "rht")
-        lay = Layout(buckets[0].numel(), self.world, bits, codec)
-        assert buckets[0].numel() <= self.max_numel
+        lay = self._layout(buckets[0].numel(), bits, codec)
+        assert lay.numel <= self.max_numel
+        self._join_streams()
         self.epoch += 1
         if preset_flags:
             for f in self.flags:
@@ -404,7 +430,11 @@ class LocalCluster:
 
     def allreduce_(self, buckets: List[torch.Tensor], bits: int, topology: str = "ring", correlated: bool = False,
                    **kw) -> List[torch.Tensor]:
-        progs = torch.stack([program_tensor(r, self.world, topology, correlated) for r in range(self.world)])
+        key = (topology, correlated)
+        progs = self._programs.get(key)
+        if progs is None:
+            progs = self._programs[key] = torch.stack([program_tensor(r, self.world, topology, correlated)
+                                                       for r in range(self.world)])
         self.run(buckets, progs, bits, **kw)
         return buckets
 
