@@ -28,6 +28,11 @@ void fused_allreduce_local(std::vector<at::Tensor> buckets, at::Tensor steps, st
                            int64_t scales_off, int64_t flag_base, int64_t epoch, int64_t seed, int64_t step,
                            int64_t bucket_id, double post_scale, int64_t timeout_ns, bool no_transmit, int64_t codec, double sc_lattice_max, double sc_c1, double sc_c2,
                      c10::optional<at::Tensor> sc_lut, c10::optional<at::Tensor> sc_plan, bool prefetch);
+std::tuple<at::Tensor, at::Tensor> rht_encode(at::Tensor x, c10::optional<at::Tensor> codes, c10::optional<at::Tensor> scales,
+                                              int64_t bits, int64_t seed, int64_t step, int64_t bucket_id, int64_t tag,
+                                              int64_t max_warps);
+void rht_decode(at::Tensor codes, at::Tensor scales, at::Tensor out, int64_t bits, int64_t seed, int64_t step,
+                int64_t bucket_id, double post_scale, int64_t max_warps);
 std::tuple<at::Tensor, at::Tensor, at::Tensor> norm_fwd(at::Tensor x, at::Tensor w, c10::optional<at::Tensor> b,
                                                         double eps, bool rms);
 std::tuple<at::Tensor, at::Tensor, at::Tensor> norm_bwd(at::Tensor dy, at::Tensor x, at::Tensor w, at::Tensor mean,
@@ -91,6 +96,10 @@ TORCH_LIBRARY(dq, m) {
         "int seed) -> ()", &dq::thc_quantize_);
   m.def("thc_dequantize_(Tensor(a!) total, Tensor stats, int world, float t_over_sqrt_d, int levels) -> ()",
         &dq::thc_dequantize_);
+  m.def("rht_encode(Tensor x, Tensor? codes, Tensor? scales, int bits, int seed, int step, int bucket_id, int tag, "
+        "int max_warps) -> (Tensor, Tensor)", &dq::rht_encode);
+  m.def("rht_decode(Tensor codes, Tensor scales, Tensor(a!) out, int bits, int seed, int step, int bucket_id, "
+        "float post_scale, int max_warps) -> ()", &dq::rht_decode);
   m.def("rope(Tensor x, Tensor cos, Tensor sin, bool backward) -> Tensor", &dq::rope);
   m.def("adamw_step(Tensor table, Tensor numel, Tensor chunk_start, int total_chunks, bool param_bf16, bool grad_bf16, "
         "float lr, float beta1, float beta2, float eps, float weight_decay, int step, float grad_scale) -> ()", &dq::adamw_step);

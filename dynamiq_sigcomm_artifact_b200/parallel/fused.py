@@ -461,15 +461,27 @@ class RhtCodec:
     """Standalone rotation-codec operators on one GPU (compress / decompress / hop).
 
     The equivalents of ``eden_utils.scaling_compress / scaling_decompress / scaling_dec_comp``
-    (cuda_kernels/src/srrcomp/eden_utils/eden_utils.cpp:133-219) for the `rht` family; each is
-    a one-step program of the fused kernel.  Messages are (code words int32 [nb, bits, 32],
-    scales fp32 [nb]).
+    (cuda_kernels/src/srrcomp/eden_utils/eden_utils.cpp:133-219) for the `rht` family.  Messages are (code words
+    int32 [nb, bits, 32], scales fp32 [nb]).  With the register rotation each is one launch that reads and writes the
+    caller's tensors (csrc/kernels/rht_codec_ops.cu), on at most `ctas` x `threads` threads; with ``rotation="tc"`` it
+    is a one-step program of the fused kernel.
     """
 
     def __init__(self, bits: int, max_numel: int, seed: int = 0, ctas: int = 32, threads: int = 256, device="cuda",
                  rotation: str = "simt"):
         self.bits, self.seed = bits, seed
         self.cluster = LocalCluster(1, max_numel, ctas=ctas, threads=threads, device=device, rotation=rotation)
+        self._max_warps = ctas * threads // 32
+
+    def _flat(self, x: torch.Tensor) -> torch.Tensor:
+        assert x.numel() <= self.cluster.max_numel
+        return x.detach().reshape(-1).contiguous()
+
+    def _message(self, msg) -> Tuple[torch.Tensor, torch.Tensor]:
+        """(codes, scales) where and as the kernel reads them (no copy for what the operators return)."""
+        codes, scales = msg
+        device = self.cluster.device
+        return codes.to(device, torch.int32).contiguous(), scales.to(device, torch.float32).contiguous()
 
     def _prog(self, step: sch.Step) -> torch.Tensor:
         return torch.tensor([[step.as_ints()]], dtype=torch.int32)
@@ -481,6 +493,9 @@ class RhtCodec:
         s.copy_(scales)
 
     def compress(self, x: torch.Tensor, step: int = 0, bucket_id: int = 0, tag: int = sch.TAG_ENCODE):
+        if not self.cluster.tensor_rotation:
+            return self.cluster.ops.rht_encode(self._flat(x), None, None, self.bits, self.seed, step, bucket_id,
+                                               tag & ~sch.TAG_STRATIFIED, self._max_warps)
         lay = Layout(x.numel(), 1, self.bits)
         work = x.detach().clone().reshape(-1)
         self.cluster.run([work], self._prog(sch.Step(shard=0, out=sch.OUT_SEND, dst=0, send_slot=0, tag=tag)),
@@ -490,15 +505,23 @@ class RhtCodec:
 
     def decompress(self, msg, numel: int, step: int = 0, bucket_id: int = 0, post_scale: float = 1.0,
                    dtype=torch.float32) -> torch.Tensor:
+        out = torch.empty(numel, dtype=dtype, device=self.cluster.device)
+        if not self.cluster.tensor_rotation:
+            assert numel <= self.cluster.max_numel
+            self.cluster.ops.rht_decode(*self._message(msg), out, self.bits, self.seed, step, bucket_id, post_scale,
+                                        self._max_warps)
+            return out
         lay = Layout(numel, 1, self.bits)
         self._put(0, msg, lay)
-        out = torch.empty(numel, dtype=dtype, device=self.cluster.device)
         self.cluster.run([out], self._prog(sch.Step(shard=0, recv_slot=0, nrecv=1, out=sch.OUT_DECODE)), self.bits,
                          seed=self.seed, step=step, bucket_id=bucket_id, post_scale=post_scale, preset_flags=True)
         return out
 
     def dec_comp(self, msg, x_local: torch.Tensor, step: int = 0, bucket_id: int = 0, tag: int = sch.TAG_ENCODE + 1):
         """decode(msg) + rotate(x_local), re-encoded: one ring hop."""
+        if not self.cluster.tensor_rotation:
+            return self.cluster.ops.rht_encode(self._flat(x_local), *self._message(msg), self.bits, self.seed, step,
+                                               bucket_id, tag & ~sch.TAG_STRATIFIED, self._max_warps)
         lay = Layout(x_local.numel(), 1, self.bits)
         self._put(0, msg, lay)
         work = x_local.detach().clone().reshape(-1)
