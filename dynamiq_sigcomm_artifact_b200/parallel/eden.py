@@ -4,9 +4,9 @@ The codec the reference inherits from its upstream package
 (cuda_kernels/src/srrcomp/srrcomp.py:293-447): a randomized Hadamard transform, 1..8-bit
 quantisation to the optimal (Lloyd-Max) levels of N(0, 1) (:364-447), bit-plane packing of the
 bins (csrc/cuda_packing.cu) and the scale ``||x||^2 / <R x, c>`` that makes the estimate unbiased
-under the random rotation.  The rotation here is blockwise over 1024 elements (the tcgen05
-kernel on GPUs); bins are packed by ``torch.ops.dq.bins_to_bits`` on GPUs and by the same plane
-layout in PyTorch on CPU.
+under the random rotation.  The rotation here is blockwise over 1024 elements.  On GPUs compress and
+decompress are one kernel each (csrc/kernels/eden_ops.cu); on CPU the same steps and the same plane
+layout are PyTorch operators.  ``pack_bins`` / ``unpack_bins`` are the packing alone.
 """
 from __future__ import annotations
 
@@ -18,6 +18,7 @@ import torch
 
 from .. import ops as _ops
 from ..ops.fwht import BLOCK, fwht1024, ifwht1024
+from ..utils import counters
 
 
 @functools.lru_cache(maxsize=None)
@@ -70,9 +71,20 @@ class Eden:
             raise ValueError("EDEN supports 1..8 bits")
         self.bits, self.seed = bits, seed
         self.centroids, self.boundaries = lloyd_max_normal(bits)
+        self._levels = {}  # device -> centroids, then boundaries
+
+    def _levels_on(self, device: torch.device) -> torch.Tensor:
+        t = self._levels.get(device)
+        if t is None:
+            t = self._levels[device] = torch.cat([self.centroids, self.boundaries]).to(device)
+        return t
 
     def compress(self, x: torch.Tensor, step: int = 0):
         n = x.numel()
+        if x.is_cuda:
+            counters.add("eden_compress")
+            flat = x.detach().reshape(-1).float().contiguous()
+            return (*_ops.require().eden_compress(flat, self._levels_on(x.device), self.bits, self.seed, step), n)
         y = fwht1024(x.reshape(-1).float(), self.seed, step, 0, signs=True, normalize=True)
         pad = (-n) % BLOCK
         yb = torch.cat([y, y.new_zeros(pad)]).view(-1, BLOCK) if pad else y.view(-1, BLOCK)
@@ -86,6 +98,10 @@ class Eden:
     def decompress(self, msg, step: int = 0) -> torch.Tensor:
         words, scale, n = msg
         nb = scale.numel()
+        if scale.is_cuda:
+            counters.add("eden_decompress")
+            return _ops.require().eden_decompress(words.to(scale.device).contiguous(), scale.contiguous(),
+                                                  self._levels_on(scale.device), n, self.bits, self.seed, step)
         bins = unpack_bins(words, self.bits, nb * BLOCK)
         y = self.centroids.to(scale.device)[bins.long()].view(nb, BLOCK) * scale.view(nb, 1)
         return ifwht1024(y.reshape(-1), self.seed, step, 0, signs=True)[:n]
