@@ -69,7 +69,9 @@ void rht_widths_update(at::Tensor mailbox, at::Tensor plan, int64_t nblocks, int
 at::Tensor rope(at::Tensor x, at::Tensor cos, at::Tensor sin, bool backward);
 void adamw_step(at::Tensor table, at::Tensor numel, at::Tensor chunk_start, int64_t total_chunks, bool param_bf16,
                 bool grad_bf16, double lr, double beta1, double beta2, double eps, double weight_decay, int64_t step,
-                double grad_scale);
+                double grad_scale, c10::optional<at::Tensor> hyper);
+void adamw_hyper(at::Tensor hyper, double lr, double beta1, double beta2, double eps, double weight_decay, int64_t step,
+                 double grad_scale);
 }  // namespace dq
 
 TORCH_LIBRARY(dq, m) {
@@ -108,7 +110,10 @@ TORCH_LIBRARY(dq, m) {
         "float post_scale, int max_warps) -> ()", &dq::rht_decode);
   m.def("rope(Tensor x, Tensor cos, Tensor sin, bool backward) -> Tensor", &dq::rope);
   m.def("adamw_step(Tensor table, Tensor numel, Tensor chunk_start, int total_chunks, bool param_bf16, bool grad_bf16, "
-        "float lr, float beta1, float beta2, float eps, float weight_decay, int step, float grad_scale) -> ()", &dq::adamw_step);
+        "float lr, float beta1, float beta2, float eps, float weight_decay, int step, float grad_scale, Tensor? hyper=None) -> ()",
+        &dq::adamw_step);
+  m.def("adamw_hyper(Tensor(a!) hyper, float lr, float beta1, float beta2, float eps, float weight_decay, int step, "
+        "float grad_scale) -> ()", &dq::adamw_hyper);
   m.def("topology() -> Tensor", &dq::topology);
   m.def("symm_alloc(int device, int bytes) -> (int, Tensor)", &dq::symm_alloc);
   m.def("symm_open(int device, Tensor handle) -> int", &dq::symm_open);

@@ -172,12 +172,21 @@ __global__ void rope_kernel(const T* __restrict__ x, const float* __restrict__ c
 // tensor t (chunk = 4096 elements).
 constexpr int kAdamChunk = 4096;
 constexpr int kAdamCols = 5;
+
+// The step's scalars.  They are launch arguments, or - for a launch inside a CUDA graph, whose arguments are frozen -
+// live in device memory, where adamw_hyper_kernel puts them before every replay.
+struct AdamHyper {
+  float lr, beta1, beta2, eps, wd, bc1, bc2, grad_scale;
+};
+__global__ void adamw_hyper_kernel(AdamHyper h, AdamHyper* out) { *out = h; }
+
 template <typename P, typename G>
 __global__ void __launch_bounds__(256) adamw_kernel(const long long* __restrict__ table,
                                                     const long long* __restrict__ numel,
-                                                    const int* __restrict__ chunk_start, int ntensors, float lr,
-                                                    float beta1, float beta2, float eps, float wd, float bc1,
-                                                    float bc2, float grad_scale) {
+                                                    const int* __restrict__ chunk_start, int ntensors,
+                                                    AdamHyper by_value, const AdamHyper* __restrict__ in_memory) {
+  const AdamHyper h = in_memory != nullptr ? *in_memory : by_value;
+  const float beta1 = h.beta1, beta2 = h.beta2, eps = h.eps, lr = h.lr, wd = h.wd, grad_scale = h.grad_scale;
   const int chunk = blockIdx.x;
   int lo = 0, hi = ntensors - 1;
   while (lo < hi) {  // last tensor whose first chunk is <= chunk
@@ -193,7 +202,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(const long long* __restrict_
   __nv_bfloat16* shadow = reinterpret_cast<__nv_bfloat16*>(table[kAdamCols * t + 4]);
   const long long n = numel[t];
   const long long base = static_cast<long long>(chunk - chunk_start[t]) * kAdamChunk;
-  const float step_size = lr / bc1, inv_bc2_sqrt = rsqrtf(bc2);
+  const float step_size = lr / h.bc1, inv_bc2_sqrt = rsqrtf(h.bc2);
   auto update = [&](float gi, float& pi, float& mi, float& vi) {
     gi *= grad_scale;
     mi = beta1 * mi + (1.f - beta1) * gi;
@@ -494,23 +503,48 @@ at::Tensor rope(at::Tensor x, at::Tensor cos, at::Tensor sin, bool backward) {
   return y;
 }
 
+namespace {
+AdamHyper adam_hyper(double lr, double beta1, double beta2, double eps, double weight_decay, int64_t step, double grad_scale) {
+  AdamHyper h;
+  h.lr = static_cast<float>(lr), h.beta1 = static_cast<float>(beta1), h.beta2 = static_cast<float>(beta2);
+  h.eps = static_cast<float>(eps), h.wd = static_cast<float>(weight_decay);
+  h.bc1 = static_cast<float>(1.0 - std::pow(beta1, static_cast<double>(step)));
+  h.bc2 = static_cast<float>(1.0 - std::pow(beta2, static_cast<double>(step)));
+  h.grad_scale = static_cast<float>(grad_scale);
+  return h;
+}
+}  // namespace
+
+// hyper: fp32 [8] device tensor that later adamw_step launches read
+void adamw_hyper(at::Tensor hyper, double lr, double beta1, double beta2, double eps, double weight_decay, int64_t step,
+                 double grad_scale) {
+  TORCH_CHECK(hyper.is_cuda() && hyper.scalar_type() == at::kFloat && hyper.is_contiguous() &&
+                  hyper.numel() * sizeof(float) >= sizeof(AdamHyper), "adamw: hyper must be 8 CUDA floats");
+  c10::cuda::CUDAGuard guard(hyper.device());
+  adamw_hyper_kernel<<<1, 1, 0, at::cuda::getCurrentCUDAStream()>>>(
+      adam_hyper(lr, beta1, beta2, eps, weight_decay, step, grad_scale), reinterpret_cast<AdamHyper*>(hyper.data_ptr<float>()));
+  C10_CUDA_KERNEL_LAUNCH_CHECK();
+}
+
 // table: int64 [T, 5] device tensor of addresses (param, grad, m, v, bf16 shadow or 0); numel: int64 [T] device; chunk_start: int32 [T] device.
+// `hyper` (fp32 [8] on the device) stands in for the scalar arguments when given.
 void adamw_step(at::Tensor table, at::Tensor numel, at::Tensor chunk_start, int64_t total_chunks, bool param_bf16,
                 bool grad_bf16, double lr, double beta1, double beta2, double eps, double weight_decay, int64_t step,
-                double grad_scale) {
+                double grad_scale, c10::optional<at::Tensor> hyper) {
   TORCH_CHECK(table.is_cuda() && table.scalar_type() == at::kLong && table.dim() == 2 && table.size(1) == kAdamCols, "adamw: bad table");
   TORCH_CHECK(numel.is_cuda() && numel.scalar_type() == at::kLong && chunk_start.is_cuda() && chunk_start.scalar_type() == at::kInt, "adamw: bad metadata");
+  TORCH_CHECK(!hyper.has_value() || (hyper->is_cuda() && hyper->scalar_type() == at::kFloat && hyper->is_contiguous() &&
+                                     hyper->numel() * sizeof(float) >= sizeof(AdamHyper)), "adamw: hyper must be 8 CUDA floats");
   if (total_chunks == 0) return;
   c10::cuda::CUDAGuard guard(table.device());
   const int T = static_cast<int>(table.size(0));
-  const float bc1 = static_cast<float>(1.0 - std::pow(beta1, static_cast<double>(step)));
-  const float bc2 = static_cast<float>(1.0 - std::pow(beta2, static_cast<double>(step)));
+  const AdamHyper h = adam_hyper(lr, beta1, beta2, eps, weight_decay, step, grad_scale);
+  const AdamHyper* hp = hyper.has_value() ? reinterpret_cast<const AdamHyper*>(hyper->data_ptr<float>()) : nullptr;
   auto stream = at::cuda::getCurrentCUDAStream();
 #define DQ_LAUNCH(P, G)                                                                                              \
   adamw_kernel<P, G><<<static_cast<unsigned>(total_chunks), 256, 0, stream>>>(                                      \
       reinterpret_cast<const long long*>(table.data_ptr<int64_t>()), reinterpret_cast<const long long*>(numel.data_ptr<int64_t>()), \
-      chunk_start.data_ptr<int>(), T, static_cast<float>(lr), static_cast<float>(beta1), static_cast<float>(beta2), \
-      static_cast<float>(eps), static_cast<float>(weight_decay), bc1, bc2, static_cast<float>(grad_scale))
+      chunk_start.data_ptr<int>(), T, h, hp)
   if (param_bf16 && grad_bf16) DQ_LAUNCH(__nv_bfloat16, __nv_bfloat16);
   else if (param_bf16) DQ_LAUNCH(__nv_bfloat16, float);
   else if (grad_bf16) DQ_LAUNCH(float, __nv_bfloat16);

@@ -82,14 +82,12 @@ def mask_tokens(input_ids: torch.Tensor, vocab: int, mask_token_id: int, generat
     """BERT masking: 15% of positions become targets; of those 80% -> [MASK], 10% -> a random
     token, 10% unchanged (testbed_evaluation/train_llm_maskedlm_bert.py:354-385)."""
     dev = input_ids.device
-    labels = input_ids.clone()
     r = torch.rand(input_ids.shape, generator=generator, device=dev)
     masked = r < mlm_probability
-    labels[~masked] = -100
     r2 = torch.rand(input_ids.shape, generator=generator, device=dev)
-    out = input_ids.clone()
-    out[masked & (r2 < 0.8)] = mask_token_id
-    rand_sel = masked & (r2 >= 0.8) & (r2 < 0.9)
     rnd = torch.randint(0, vocab, input_ids.shape, generator=generator, device=dev)
-    out[rand_sel] = rnd[rand_sel]
+    # elementwise selections: an assignment through a boolean mask would wait for the mask's count on the host
+    labels = torch.where(masked, input_ids, -100)
+    out = torch.where(masked & (r2 < 0.8), mask_token_id, input_ids)
+    out = torch.where(masked & (r2 >= 0.8) & (r2 < 0.9), rnd, out)
     return out, labels

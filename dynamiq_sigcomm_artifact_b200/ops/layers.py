@@ -200,6 +200,28 @@ class FusedAdamW(torch.optim.Optimizer):
         self._tables = {}
         self._step = 0
         self._shadows = dict(shadows or {})
+        self.use_hyper = False  # True while a step is captured: launches read the scalars from device memory
+        self._hyper: Optional[torch.Tensor] = None
+        self.generation = 0  # moves when the state tensors are replaced
+
+    def hyper(self, device) -> torch.Tensor:
+        """The step's scalars on the device, for launches inside a CUDA graph."""
+        if self._hyper is None:
+            self._hyper = torch.zeros(8, dtype=torch.float32, device=device)
+        return self._hyper
+
+    def write_hyper(self, grad_scale: float = 1.0) -> None:
+        """Put this step's scalars (of the only parameter group) where a captured step reads them."""
+        group = self.param_groups[0]
+        b1, b2 = group["betas"]
+        require().adamw_hyper(self._hyper, group["lr"], b1, b2, group["eps"], group["weight_decay"], self._step, grad_scale)
+        counters.add("adamw_hyper")
+
+    def prepare_subset(self, key, params: List[torch.Tensor]) -> None:
+        """State and pointer table of a subset that :meth:`step_params` will update (nothing is updated)."""
+        if params and params[0].is_cuda:
+            self.hyper(params[0].device)
+            self._table(("subset", key), {"params": params})
 
     def _table(self, gi, group) -> list:
         """Per (param dtype, grad dtype) metadata; rebuilt when a gradient buffer moves.  `gi` is any
@@ -263,7 +285,7 @@ class FusedAdamW(torch.optim.Optimizer):
             ops = require()
             for table, numel, starts, chunks, pbf, gbf, _ in self._table(("subset", key), {"params": params}):
                 ops.adamw_step(table, numel, starts, chunks, pbf, gbf, group["lr"], b1, b2, group["eps"],
-                               group["weight_decay"], self._step, grad_scale)
+                               group["weight_decay"], self._step, grad_scale, self._hyper if self.use_hyper else None)
                 counters.add("adamw")
         else:
             self._step_cpu([p for p in params if p.grad is not None], group, grad_scale)
@@ -322,3 +344,4 @@ class FusedAdamW(torch.optim.Optimizer):
         self._step = d.pop("fused_step", 0)
         super().load_state_dict(d)
         self._tables.clear()
+        self.generation += 1

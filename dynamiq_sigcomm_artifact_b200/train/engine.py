@@ -74,7 +74,7 @@ class TrainConfig:
     comm_prefetch: bool = True  # staging buffer of the collective kernel (off: half the shared memory per CTA)
     warmup_steps: int = 2
     measure_comm_error: bool = False
-    cuda_graphs: bool = True  # capture each transformer block's forward and backward as CUDA graphs
+    cuda_graphs: bool = True  # one GPU: capture the whole step (train/step_graph.py); several: each transformer block
     reducer: str = "flat"  # "flat": gradient arena + bucket pipeline of this package; "ddp": torch DDP + comm hook
     sparse_embedding: Optional[bool] = None  # True: tied-embedding lookup gradient exchanged as token rows
 
@@ -128,7 +128,7 @@ class Trainer:
                 self.reducer.broadcast_parameters(0)
                 if self.shadows:
                     enable_shadows(self.model)
-            if use_graphs:
+            if use_graphs and self.world > 1:
                 self.graphed = self._graph_blocks()
             self.reducer.arena.zero_()
             self.reducer.install_marks()
@@ -152,6 +152,56 @@ class Trainer:
         self._gen = torch.Generator(device=device).manual_seed(cfg.seed + 17 * self.rank + 1) \
             if device.type == "cuda" else torch.Generator().manual_seed(cfg.seed + 17 * self.rank + 1)
         self.autocast_dtype = {"bf16": torch.bfloat16, "fp32": None}[cfg.dtype]
+        # whole-step graphs by (shape, dtype, labels given); None: seen once, captured when it comes again
+        self._graph_step = use_graphs and self.world == 1 and self.reducer is not None
+        self._step_graphs: dict = {}
+        self._graph_pool = None
+        if self._graph_step:
+            ids = torch.zeros(cfg.micro_batch, cfg.seq_len, dtype=torch.int64, device=device)
+            self._capture_step(self._step_key(ids, None), ids, None)
+            self.graphed = self._graph_step
+
+    MAX_STEP_GRAPHS = 4  # captured input shapes; further shapes run eagerly
+
+    @staticmethod
+    def _step_key(ids: torch.Tensor, labels: Optional[torch.Tensor]) -> tuple:
+        return (tuple(ids.shape), ids.dtype, None if labels is None else (tuple(labels.shape), labels.dtype))
+
+    def _graph_addresses(self) -> tuple:
+        """What a captured step has baked in and a caller could move."""
+        return (self.opt.generation, *[p.data_ptr() for p in self._params])
+
+    def _capture_step(self, key: tuple, ids: torch.Tensor, labels: Optional[torch.Tensor]):
+        from .step_graph import StepGraph
+
+        self._params = list(self.model.parameters())
+        if self._graph_pool is None:
+            self._graph_pool = torch.cuda.graph_pool_handle()
+        try:
+            self._step_graphs[key] = StepGraph(self, ids, labels, self._graph_pool)
+        except torch.cuda.OutOfMemoryError:
+            raise
+        except Exception as e:  # fall back to eager execution, loudly
+            print(f"[dynamiq] CUDA graph capture of the step failed ({type(e).__name__}: {e}); running eagerly", flush=True)
+            self._graph_step = False
+            return None
+        return self._step_graphs[key]
+
+    def _step_graph(self, ids: torch.Tensor, labels: Optional[torch.Tensor]):
+        """The captured step for these inputs, or None to run it eagerly."""
+        if not (self._graph_step and self.model.training and len(self.opt.param_groups) == 1):
+            return None
+        key = self._step_key(ids, labels)
+        g = self._step_graphs.get(key)
+        if g is not None and g.addresses != self._graph_addresses():
+            self._step_graphs.clear()  # parameters or optimizer state moved: every graph is stale
+            g = self._step_graphs[key] = None
+        if g is None:
+            if key in self._step_graphs:
+                g = self._capture_step(key, ids, labels)
+            elif len(self._step_graphs) < self.MAX_STEP_GRAPHS:
+                self._step_graphs[key] = None
+        return g
 
     def _graph_blocks(self) -> bool:
         """Capture every transformer block (forward and backward) as CUDA graphs: a step then issues
@@ -210,48 +260,65 @@ class Trainer:
             off += p.numel()
 
     # -- one step ------------------------------------------------------------------------
-    def train_step_device(self, input_ids: torch.Tensor, labels: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """One optimizer step on device-resident token ids; returns the loss tensor (no sync)."""
-        cfg = self.cfg
-        if self.state is not None:
-            self.state.begin_step(self.step_idx)
-        if cfg.task == "mlm" and labels is None:
+    def _forward_backward(self, input_ids: torch.Tensor, labels: Optional[torch.Tensor]) -> torch.Tensor:
+        """Forward and backward with the bucket pipeline (hooks and optimizer steps included); returns the loss."""
+        if self.cfg.task == "mlm" and labels is None:
             c = self.model.config
             input_ids, labels = mask_tokens(input_ids, c.vocab, c.mask_token_id, self._gen)
         elif labels is None:
             labels = input_ids
         if self.autocast_dtype is not None and self.device.type == "cuda":
-            with torch.autocast("cuda", dtype=self.autocast_dtype):
+            # with one use of every weight per step a cache of casts has nothing to reuse
+            with torch.autocast("cuda", dtype=self.autocast_dtype, cache_enabled=False):
                 loss = self.net(input_ids, labels)
         else:
             loss = self.net(input_ids, labels)
         if self.reducer is not None:
-            self.opt.advance()
             self.reducer.begin_step()
         loss.backward()
-        if self.graphed:
-            from ..utils import counters
-
-            counters.add("graphed_blocks", self._launches_per_graphed_step)
         if self.reducer is not None:
             self.reducer.finish()  # every bucket: hook, then its AdamW step, on the side stream
-            self.sched.step()
+        return loss.detach()
+
+    def _step(self, input_ids: torch.Tensor, labels: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """One optimizer step; the loss may live in a buffer that the next step overwrites."""
+        if self.state is not None:
+            self.state.begin_step(self.step_idx)
+        graph = self._step_graph(input_ids, labels)
+        if self.reducer is not None:
+            self.opt.advance()
+        if graph is not None:
+            self.opt.write_hyper()
+            loss = graph.run(input_ids, labels)
         else:
+            input_ids = input_ids.to(self.device, non_blocking=True)
+            if labels is not None:
+                labels = labels.to(self.device, non_blocking=True)
+            loss = self._forward_backward(input_ids, labels)
+            if self.graphed and self.world > 1:
+                from ..utils import counters
+
+                counters.add("graphed_blocks", self._launches_per_graphed_step)
+        if self.reducer is None:
             self.opt.step()
-            self.sched.step()
+        self.sched.step()
+        if self.reducer is None:
             if self.ddp is None:
                 self._flat_grad.zero_()
             else:
                 self.opt.zero_grad(set_to_none=False)
         self.step_idx += 1
         self._poll_status(enqueue=True)
-        return loss.detach()
+        return loss
+
+    def train_step_device(self, input_ids: torch.Tensor, labels: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """One optimizer step on device-resident token ids; returns the loss tensor (no sync)."""
+        loss = self._step(input_ids, labels)
+        return loss.clone() if self._graph_step else loss
 
     def train_step(self, input_ids_host: torch.Tensor, labels_host: Optional[torch.Tensor] = None) -> float:
         """Public API: host batch in, loss out.  Copies the batch to the device every call."""
-        ids = input_ids_host.to(self.device, non_blocking=True)
-        lab = labels_host.to(self.device, non_blocking=True) if labels_host is not None else None
-        loss = float(self.train_step_device(ids, lab).item())
+        loss = float(self._step(input_ids_host, labels_host).item())
         self._poll_status(enqueue=False)  # the loss read-back synchronised: this step's status copy has landed
         return loss
 

@@ -14,3 +14,12 @@ def total() -> int:
 
 def reset() -> None:
     LAUNCHES.clear()
+
+
+def snapshot() -> Counter:
+    return Counter(LAUNCHES)
+
+
+def restore(saved: Counter) -> None:
+    LAUNCHES.clear()
+    LAUNCHES.update(saved)
