@@ -51,6 +51,14 @@ at::Tensor swiglu_fwd(at::Tensor in);
 at::Tensor swiglu_bwd(at::Tensor dy, at::Tensor in);
 std::tuple<at::Tensor, at::Tensor> superchunk_center(at::Tensor x, int64_t world);
 void superchunk_add_mean(at::Tensor resid, at::Tensor mean, at::Tensor out);
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_fwd(at::Tensor x, c10::optional<at::Tensor> delta,
+                                                                        c10::optional<at::Tensor> bias, at::Tensor w,
+                                                                        c10::optional<at::Tensor> b, double eps, bool rms);
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_bwd(
+    at::Tensor dy, c10::optional<at::Tensor> dy2, c10::optional<at::Tensor> ds, at::Tensor s, at::Tensor w, at::Tensor mean,
+    at::Tensor rstd, bool rms, bool want_bias, c10::optional<at::Tensor> dw_out, c10::optional<at::Tensor> db_out,
+    c10::optional<at::Tensor> dbias_out);
+at::Tensor residual_add(at::Tensor x, at::Tensor delta, c10::optional<at::Tensor> bias);
 std::tuple<at::Tensor, at::Tensor> eden_compress(at::Tensor x, at::Tensor levels, int64_t bits, int64_t seed, int64_t step);
 at::Tensor eden_decompress(at::Tensor words, at::Tensor scale, at::Tensor levels, int64_t n, int64_t bits, int64_t seed,
                            int64_t step);
@@ -88,6 +96,12 @@ TORCH_LIBRARY(dq, m) {
   m.def("swiglu_bwd(Tensor dy, Tensor x) -> Tensor", &dq::swiglu_bwd);
   m.def("superchunk_center(Tensor x, int world) -> (Tensor, Tensor)", &dq::superchunk_center);
   m.def("superchunk_add_mean(Tensor resid, Tensor mean, Tensor(a!) out) -> ()", &dq::superchunk_add_mean);
+  m.def("add_norm_fwd(Tensor x, Tensor? delta, Tensor? bias, Tensor w, Tensor? b, float eps, bool rms) -> (Tensor, Tensor, Tensor, Tensor)",
+        &dq::add_norm_fwd);
+  m.def("add_norm_bwd(Tensor dy, Tensor? dy2, Tensor? ds, Tensor s, Tensor w, Tensor mean, Tensor rstd, bool rms, bool want_bias, "
+        "Tensor(a!)? dw_out=None, Tensor(b!)? db_out=None, Tensor(c!)? dbias_out=None) -> (Tensor, Tensor, Tensor, Tensor)",
+        &dq::add_norm_bwd);
+  m.def("residual_add(Tensor x, Tensor delta, Tensor? bias) -> Tensor", &dq::residual_add);
   m.def("eden_compress(Tensor x, Tensor levels, int bits, int seed, int step) -> (Tensor, Tensor)", &dq::eden_compress);
   m.def("eden_decompress(Tensor words, Tensor scale, Tensor levels, int n, int bits, int seed, int step) -> Tensor",
         &dq::eden_decompress);

@@ -6,7 +6,7 @@
  * the RMSNorm backward pass - a host without the PyTorch caching allocator (a plain C/C++ or
  * ctypes caller), a caller running under a fixed memory budget that was carved up in advance,
  * or a real-time loop where a cudaMalloc (which synchronises the device) is not acceptable.
- * The regular operator (torch.ops.dq.norm_bwd) asks the allocator for its per-warp partial-sum
+ * The regular operator (torch.ops.dq.norm_bwd) asks the allocator for its partial-sum
  * scratch on every call; this variant keeps that scratch in a fixed array inside the library.
  *
  * The scratch is a file-scope device array of DQ_NOALLOC_MAX_PARTS x DQ_NOALLOC_MAX_HIDDEN

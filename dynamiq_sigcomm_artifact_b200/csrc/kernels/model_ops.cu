@@ -13,6 +13,16 @@
 
 namespace dq {
 
+// residual_norm.cu: rows of up to 2048 columns
+bool norm_rows_fit(int64_t H);
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_fwd(at::Tensor x, c10::optional<at::Tensor> delta,
+                                                                        c10::optional<at::Tensor> bias, at::Tensor w,
+                                                                        c10::optional<at::Tensor> b, double eps, bool rms);
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_bwd(
+    at::Tensor dy, c10::optional<at::Tensor> dy2, c10::optional<at::Tensor> ds, at::Tensor s, at::Tensor w, at::Tensor mean,
+    at::Tensor rstd, bool rms, bool want_bias, c10::optional<at::Tensor> dw_out, c10::optional<at::Tensor> db_out,
+    c10::optional<at::Tensor> dbias_out);
+
 namespace {
 
 using namespace normk;
@@ -333,6 +343,10 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> norm_fwd(at::Tensor x, at::Tensor
   check_norm_inputs(x, w);
   c10::cuda::CUDAGuard guard(x.device());
   const int H = static_cast<int>(x.size(-1));
+  if (norm_rows_fit(H)) {
+    auto out = add_norm_fwd(x, c10::nullopt, c10::nullopt, w, b, eps, rms);
+    return {std::get<1>(out), std::get<2>(out), std::get<3>(out)};
+  }
   const int rows = static_cast<int>(x.numel() / H);
   at::Tensor y = at::empty_like(x);
   auto fopt = x.options().dtype(at::kFloat);
@@ -366,6 +380,10 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> norm_bwd(at::Tensor dy, at::Tenso
   TORCH_CHECK(dy.is_contiguous() && dy.scalar_type() == x.scalar_type() && dy.numel() == x.numel(), "norm_bwd: dy/x mismatch");
   c10::cuda::CUDAGuard guard(x.device());
   const int H = static_cast<int>(x.size(-1));
+  if (norm_rows_fit(H)) {
+    auto out = add_norm_bwd(dy, c10::nullopt, c10::nullopt, x, w, mean, rstd, rms, false, dw_out, db_out, c10::nullopt);
+    return {std::get<0>(out), std::get<1>(out), std::get<2>(out)};
+  }
   const int rows = static_cast<int>(x.numel() / H);
   at::Tensor dx = at::empty_like(x);
   auto fopt = x.options().dtype(at::kFloat);
@@ -378,43 +396,6 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> norm_bwd(at::Tensor dy, at::Tenso
   };
   at::Tensor dw = usable(dw_out) ? *dw_out : at::empty({H}, fopt);
   at::Tensor db = rms ? at::empty({0}, fopt) : (usable(db_out) ? *db_out : at::empty({H}, fopt));
-  if (H <= 2048) {
-    const int grid = std::max(1, std::min((rows + kNormWarps - 1) / kNormWarps, 2 * sm_count()));
-    const int nparts = grid * kNormWarps;
-    at::Tensor dw_part = at::empty({nparts, H}, fopt), db_part = at::empty({rms ? 0 : nparts, H}, fopt);
-    const int nchunk = (H + 255) / 256;
-#define DQ_ROWS(T, RMS, NC)                                                                                        \
-  norm_bwd_rows_kernel<T, RMS, NC><<<grid, kNormWarps * 32, 0, stream>>>(                                          \
-      reinterpret_cast<const T*>(dy.data_ptr()), reinterpret_cast<const T*>(x.data_ptr()), w.data_ptr<float>(),    \
-      rms ? nullptr : mean.data_ptr<float>(), rstd.data_ptr<float>(), reinterpret_cast<T*>(dx.data_ptr()),         \
-      dw_part.data_ptr<float>(), rms ? nullptr : db_part.data_ptr<float>(), rows, H)
-#define DQ_ROWS_NC(T, RMS)                                 \
-  switch (nchunk) {                                        \
-    case 1: DQ_ROWS(T, RMS, 1); break;                     \
-    case 2: DQ_ROWS(T, RMS, 2); break;                     \
-    case 3: DQ_ROWS(T, RMS, 3); break;                     \
-    case 4: DQ_ROWS(T, RMS, 4); break;                     \
-    case 5: case 6: DQ_ROWS(T, RMS, 6); break;             \
-    default: DQ_ROWS(T, RMS, 8); break;                    \
-  }
-    if (x.scalar_type() == at::kBFloat16) {
-      if (rms) { DQ_ROWS_NC(__nv_bfloat16, true) } else { DQ_ROWS_NC(__nv_bfloat16, false) }
-    } else {
-      if (rms) { DQ_ROWS_NC(float, true) } else { DQ_ROWS_NC(float, false) }
-    }
-#undef DQ_ROWS_NC
-#undef DQ_ROWS
-    C10_CUDA_KERNEL_LAUNCH_CHECK();
-    dim3 rb(32, 32);
-    if (rms)
-      reduce_parts2_kernel<<<(H + 31) / 32, rb, 0, stream>>>(dw_part.data_ptr<float>(), dw.data_ptr<float>(), nparts, H);
-    else
-      reduce_parts2_pair_kernel<<<dim3((H + 31) / 32, 2), rb, 0, stream>>>(dw_part.data_ptr<float>(), dw.data_ptr<float>(),
-                                                                           db_part.data_ptr<float>(), db.data_ptr<float>(),
-                                                                           nparts, H);
-    C10_CUDA_KERNEL_LAUNCH_CHECK();
-    return {dx, dw, db};
-  }
   const int grid = std::max(1, std::min((rows + kNormWarps - 1) / kNormWarps, sm_count() * 2));
   at::Tensor dw_part = at::empty({grid, H}, fopt), db_part = at::empty({rms ? 0 : grid, H}, fopt);
   const size_t smem = static_cast<size_t>(rms ? 1 : 2) * H * sizeof(float);

@@ -1,5 +1,5 @@
 // RMSNorm backward without any allocation: the same kernels as torch.ops.dq.norm_bwd, with the
-// per-warp partial sums of dw kept in a fixed device array of this library instead of a tensor
+// per-CTA partial sums of dw kept in a fixed device array of this library instead of a tensor
 // obtained from the allocator.  Declaration and usage rules: dq_noalloc.h.  There is no
 // counterpart of this entry point in the reference implementation.
 #include "dq_noalloc.h"
@@ -10,12 +10,13 @@
 #include <cstdint>
 #include <mutex>
 
+#include "column_sums.cuh"
 #include "norm_kernels.cuh"
 
 namespace {
 
 // Scratch shared by every call on a device: [DQ_NOALLOC_MAX_PARTS][hidden] floats, fully
-// rewritten by norm_bwd_rows_kernel before reduce_parts2_kernel reads it.
+// rewritten by add_norm_bwd_kernel before reduce_arrays_kernel reads it.
 static __device__ __align__(256) float g_noalloc_scratch[DQ_NOALLOC_MAX_PARTS * DQ_NOALLOC_MAX_HIDDEN];
 
 constexpr int kMaxDevices = 64;
@@ -46,27 +47,14 @@ int scratch_for_current_device(float** out) {
   return DQ_NOALLOC_OK;
 }
 
-template <typename T, int NC>
+template <typename T>
 void launch_rows(const void* dy, const void* x, const float* w, const float* rstd, void* dx, float* parts, int rows,
                  int hidden, int grid, cudaStream_t stream) {
   using namespace dq::normk;
-  norm_bwd_rows_kernel<T, true, NC><<<grid, kNormWarps * 32, 0, stream>>>(
-      static_cast<const T*>(dy), static_cast<const T*>(x), w, nullptr, rstd, static_cast<T*>(dx), parts, nullptr, rows,
-      hidden);
-}
-
-template <typename T>
-void launch_rows_nc(int nchunk, const void* dy, const void* x, const float* w, const float* rstd, void* dx,
-                    float* parts, int rows, int hidden, int grid, cudaStream_t stream) {
-  switch (nchunk) {
-    case 1: launch_rows<T, 1>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream); break;
-    case 2: launch_rows<T, 2>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream); break;
-    case 3: launch_rows<T, 3>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream); break;
-    case 4: launch_rows<T, 4>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream); break;
-    case 5:
-    case 6: launch_rows<T, 6>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream); break;
-    default: launch_rows<T, 8>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream); break;
-  }
+  const int nt = norm_group_threads(hidden);
+  add_norm_bwd_kernel<T, true, false><<<grid, nt * norm_groups(hidden), norm_bwd_smem(hidden), stream>>>(
+      static_cast<const T*>(dy), nullptr, false, static_cast<const T*>(x), w, nullptr, rstd, static_cast<T*>(dx), parts,
+      rows, hidden, nt);
 }
 
 bool bad_ptr(const void* p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15u) != 0; }
@@ -85,15 +73,12 @@ extern "C" int dq_rmsnorm_bwd_noalloc(const void* dy, const void* x, const float
   if (rc != DQ_NOALLOC_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   (void)cudaGetLastError();  // an error left behind by the caller's earlier launches is not this call's
-  const int max_grid = DQ_NOALLOC_MAX_PARTS / kNormWarps;
-  int grid = (rows + kNormWarps - 1) / kNormWarps;
-  if (grid > max_grid) grid = max_grid;
-  const int nparts = grid * kNormWarps;  // <= DQ_NOALLOC_MAX_PARTS rows of `hidden` floats
-  const int nchunk = (hidden + 255) / 256;
-  if (is_bf16) launch_rows_nc<__nv_bfloat16>(nchunk, dy, x, w, rstd, dx, parts, rows, hidden, grid, stream);
-  else launch_rows_nc<float>(nchunk, dy, x, w, rstd, dx, parts, rows, hidden, grid, stream);
+  int grid = norm_bwd_grid(rows, hidden, dq::device_sms());  // one partial row of `hidden` floats per CTA
+  if (grid > DQ_NOALLOC_MAX_PARTS) grid = DQ_NOALLOC_MAX_PARTS;
+  if (is_bf16) launch_rows<__nv_bfloat16>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream);
+  else launch_rows<float>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream);
   dim3 rb(32, 32);
-  reduce_parts2_kernel<<<(hidden + 31) / 32, rb, 0, stream>>>(parts, dw, nparts, hidden);
+  dq::reduce_arrays_kernel<<<(hidden + 31) / 32, rb, 0, stream>>>(parts, dw, nullptr, nullptr, grid, hidden);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     t_last_cuda_error = static_cast<int>(e);

@@ -1,5 +1,5 @@
-// Kernel templates of the normalisation backward pass shared by the operator in model_ops.cu
-// and the allocation-free C entry point in norm_bwd_noalloc.cu.
+// Vector access helpers of the model kernels, and the normalisation backward kernel for rows of up to 2048 columns, shared
+// by the operators in residual_norm.cu and the allocation-free C entry point in norm_bwd_noalloc.cu.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -64,117 +64,158 @@ __device__ __forceinline__ float warp_sum(float v) {
 constexpr int kNormWarps = 8;
 
 
-// Fast path for H <= 2048: lane owns columns lane*8 + 256*i.  Each warp walks its rows once for
-// the row statistics and once more (L1-resident) for dx, accumulating its share of dw / db in
-// registers; per-warp partial sums go to dw_part[warp] and are reduced by a second kernel in a
-// fixed order.
-template <typename T, bool RMS, int NCHUNK>
-__global__ void __launch_bounds__(kNormWarps * 32) norm_bwd_rows_kernel(
-    const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ mean,
-    const float* __restrict__ rstd, T* __restrict__ dx, float* __restrict__ dw_part, float* __restrict__ db_part,
-    int rows, int H) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gw = blockIdx.x * kNormWarps + warp, nw = gridDim.x * kNormWarps;
-  float adw[NCHUNK][8], adb[RMS ? 1 : NCHUNK][8];
+// eight values as they are in memory: loads of several tensors are in flight before any of them is used
+template <typename T>
+struct Raw8;
+template <>
+struct Raw8<__nv_bfloat16> {
+  uint4 q;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { q = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void get(float (&o)[8]) const {
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-  for (int i = 0; i < NCHUNK; ++i)
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      adw[i][k] = 0.f;
-      if (!RMS) adb[i][k] = 0.f;
+    for (int i = 0; i < 4; ++i) {
+      o[2 * i] = __uint_as_float(w[i] << 16);
+      o[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
     }
-  for (int row = gw; row < rows; row += nw) {
-    const T* xr = x + static_cast<size_t>(row) * H;
-    const T* dr = dy + static_cast<size_t>(row) * H;
-    const float mu = RMS ? 0.f : mean[row], rs = rstd[row];
+  }
+};
+template <>
+struct Raw8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* p) {
+    a = *reinterpret_cast<const float4*>(p);
+    b = *reinterpret_cast<const float4*>(p + 4);
+  }
+  __device__ __forceinline__ void get(float (&o)[8]) const {
+    o[0] = a.x, o[1] = a.y, o[2] = a.z, o[3] = a.w, o[4] = b.x, o[5] = b.y, o[6] = b.z, o[7] = b.w;
+  }
+};
+
+// ---- backward of rows with H <= 2048 ----
+// A CTA holds several groups of NT threads (a multiple of 32, at least H / 8), one row per group at a time and eight
+// columns per thread, so that the column sums of dw, db and dbias are 8 registers each; a group synchronises once a row
+// on a barrier of its own, and its next row is already in flight.  At the end the groups add their sums in a fixed order
+// in shared memory and the CTA leaves one partial row: part[arrays][gridDim.x][H], arrays = dw, (db), (dbias).
+// `extra` (may be null): a second term of dy, or one of dx.
+constexpr int kNormBwdThreads = 384;  // two CTAs per SM at 80 registers
+
+inline int norm_group_threads(int H) { return (H / 8 + 31) / 32 * 32; }
+inline int norm_groups(int H) { return kNormBwdThreads / norm_group_threads(H) < 8 ? kNormBwdThreads / norm_group_threads(H) : 8; }
+inline size_t norm_bwd_smem(int H) { return static_cast<size_t>(H) * sizeof(float); }
+inline int norm_bwd_grid(int rows, int H, int sms) {
+  const int groups = norm_groups(H), want = (rows + groups - 1) / groups;
+  const int most = sms * (768 / (groups * norm_group_threads(H)));
+  return want < most ? (want > 0 ? want : 1) : most;
+}
+
+template <typename T, bool RMS, bool BIAS>
+__global__ void __launch_bounds__(kNormBwdThreads, 2) add_norm_bwd_kernel(
+    const T* __restrict__ dy, const T* __restrict__ extra, bool extra_is_dy, const T* __restrict__ s,
+    const float* __restrict__ w, const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
+    float* __restrict__ part, int rows, int H, int NT) {
+  extern __shared__ float sm[];                    // [H]
+  __shared__ float2 red[2][kNormBwdThreads / 32];  // per warp, two rows in turn
+  const int groups = blockDim.x / NT, group = threadIdx.x / NT, t = threadIdx.x - group * NT, c = t * 8;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gw = NT / 32;
+  const bool on = c < H;
+  const float inv_h = 1.0f / static_cast<float>(H);
+  float adw[8], adb[8], abias[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) adw[k] = adb[k] = abias[k] = 0.f;
+  Raw8<T> rv, rd, re, nv, nd, ne;
+  float mu = 0.f, rs = 0.f, nmu = 0.f, nrs = 0.f;
+  auto fetch = [&](int row, Raw8<T>& v, Raw8<T>& d, Raw8<T>& e, float& m, float& q) {
+    const size_t at = static_cast<size_t>(row) * H + c;
+    m = RMS ? 0.f : mean[row];
+    q = rstd[row];
+    if (on) {
+      v.load(s + at);
+      d.load(dy + at);
+      if (extra != nullptr) e.load(extra + at);
+    }
+  };
+  const int step = gridDim.x * groups;
+  int row = blockIdx.x * groups + group, turn = 0;
+  if (row < rows) fetch(row, rv, rd, re, mu, rs);
+  for (; row < rows; row += step, turn ^= 1) {
+    if (row + step < rows) fetch(row + step, nv, nd, ne, nmu, nrs);
+    // unpacked before and again after the barrier: fewer registers stay live across it
+    auto unpack = [&](float (&v)[8], float (&d)[8], float (&g)[8]) {
+      rv.get(v);
+      rd.get(d);
+      if (extra != nullptr && extra_is_dy) {
+        float e[8];
+        re.get(e);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) d[k] += e[k];
+      }
+      Vec8<float>::load(w + c, g);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = (v[k] - mu) * rs;  // normalised input
+    };
     float s1 = 0.f, s2 = 0.f;
+    if (on) {
+      float v[8], d[8], g[8];
+      unpack(v, d, g);
 #pragma unroll
-    for (int i = 0; i < NCHUNK; ++i) {
-      const int c = lane * 8 + 256 * i;
-      if (c < H) {
-        float v[8], d[8], g[8];
-        Vec8<T>::load(xr + c, v);
-        Vec8<T>::load(dr + c, d);
-        Vec8<float>::load(w + c, g);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float gdy = g[k] * d[k];
-          s1 += gdy;
-          s2 += gdy * (v[k] - mu) * rs;
-        }
+      for (int k = 0; k < 8; ++k) {
+        const float gdy = g[k] * d[k];
+        s1 += gdy;
+        s2 += gdy * v[k];
+        adw[k] += d[k] * v[k];
+        if (!RMS) adb[k] += d[k];
       }
     }
-    s1 = warp_sum(s1), s2 = warp_sum(s2);
-    const float m1 = RMS ? 0.f : s1 / H, m2 = s2 / H;
-    T* dxr = dx + static_cast<size_t>(row) * H;
-#pragma unroll
-    for (int i = 0; i < NCHUNK; ++i) {
-      const int c = lane * 8 + 256 * i;
-      if (c < H) {
-        float v[8], d[8], g[8], o[8];
-        Vec8<T>::load(xr + c, v);
-        Vec8<T>::load(dr + c, d);
-        Vec8<float>::load(w + c, g);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float xhat = (v[k] - mu) * rs;
-          o[k] = rs * (g[k] * d[k] - m1 - xhat * m2);
-          adw[i][k] += d[k] * xhat;
-          if (!RMS) adb[i][k] += d[k];
-        }
-        Vec8<T>::store(dxr + c, o);
+    if (!RMS) s1 = warp_sum(s1);
+    s2 = warp_sum(s2);
+    if (gw > 1) {
+      if (lane == 0) red[turn][warp] = make_float2(s1, s2);
+      asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(NT) : "memory");
+      s1 = s2 = 0.f;
+      for (int q = 0; q < gw; ++q) {
+        const float2 p = red[turn][group * gw + q];
+        s1 += p.x, s2 += p.y;
       }
     }
-  }
+    if (on) {
+      const float m1 = RMS ? 0.f : s1 * inv_h, m2 = s2 * inv_h;
+      float o[8], v[8], d[8], g[8];
+      unpack(v, d, g);
 #pragma unroll
-  for (int i = 0; i < NCHUNK; ++i) {
-    const int c = lane * 8 + 256 * i;
-    if (c < H) {
-      Vec8<float>::store(dw_part + static_cast<size_t>(gw) * H + c, adw[i]);
-      if (!RMS) Vec8<float>::store(db_part + static_cast<size_t>(gw) * H + c, adb[i]);
+      for (int k = 0; k < 8; ++k) o[k] = rs * (g[k] * d[k] - m1 - v[k] * m2);
+      if (extra != nullptr && !extra_is_dy) {
+        float r[8];
+        re.get(r);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) o[k] += r[k];
+      }
+      if (BIAS) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) abias[k] += o[k];
+      }
+      Vec8<T>::store(dx + static_cast<size_t>(row) * H + c, o);
     }
+    rv = nv, rd = nd, re = ne, mu = nmu, rs = nrs;
   }
-}
-
-// out[c] = sum over parts; 32 row-groups per CTA (block 32 x 32) combined through shared memory in a
-// fixed order, so the result does not depend on scheduling
-static __global__ void __launch_bounds__(1024) reduce_parts2_kernel(const float* __restrict__ part,
-                                                                    float* __restrict__ out, int nparts, int H) {
-  __shared__ float sm[32][33];
-  const int c = blockIdx.x * 32 + threadIdx.x, g = threadIdx.y;
-  float s = 0.f;
-  if (c < H)
-    for (int p = g; p < nparts; p += 32) s += part[static_cast<size_t>(p) * H + c];
-  sm[g][threadIdx.x] = s;
-  __syncthreads();
-  if (g == 0 && c < H) {
-    float t = 0.f;
+  auto combine = [&](float (&acc)[8], int array) {
+    for (int q = 0; q < groups; ++q) {
+      __syncthreads();
+      if (q == group && on) {
+        if (q > 0) {
+          float o[8];
+          Vec8<float>::load(sm + c, o);
 #pragma unroll
-    for (int k = 0; k < 32; ++k) t += sm[k][threadIdx.x];
-    out[c] = t;
-  }
-}
-
-// the same reduction for two partial-sum arrays (weight and bias gradient) in one launch: blockIdx.y picks the pair
-static __global__ void __launch_bounds__(1024) reduce_parts2_pair_kernel(const float* __restrict__ part_a,
-                                                                         float* __restrict__ out_a,
-                                                                         const float* __restrict__ part_b,
-                                                                         float* __restrict__ out_b, int nparts, int H) {
-  __shared__ float sm[32][33];
-  const float* part = blockIdx.y == 0 ? part_a : part_b;
-  float* out = blockIdx.y == 0 ? out_a : out_b;
-  const int c = blockIdx.x * 32 + threadIdx.x, g = threadIdx.y;
-  float s = 0.f;
-  if (c < H)
-    for (int p = g; p < nparts; p += 32) s += part[static_cast<size_t>(p) * H + c];
-  sm[g][threadIdx.x] = s;
-  __syncthreads();
-  if (g == 0 && c < H) {
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < 32; ++k) t += sm[k][threadIdx.x];
-    out[c] = t;
-  }
+          for (int k = 0; k < 8; ++k) acc[k] += o[k];
+        }
+        if (q == groups - 1) Vec8<float>::store(part + (static_cast<size_t>(array) * gridDim.x + blockIdx.x) * H + c, acc);
+        else Vec8<float>::store(sm + c, acc);
+      }
+    }
+  };
+  combine(adw, 0);
+  if constexpr (!RMS) combine(adb, 1);
+  if constexpr (BIAS) combine(abias, RMS ? 1 : 2);
 }
 
 }  // namespace normk
