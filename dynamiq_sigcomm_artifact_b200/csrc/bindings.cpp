@@ -59,6 +59,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_bwd(
     at::Tensor rstd, bool rms, bool want_bias, c10::optional<at::Tensor> dw_out, c10::optional<at::Tensor> db_out,
     c10::optional<at::Tensor> dbias_out);
 at::Tensor residual_add(at::Tensor x, at::Tensor delta, c10::optional<at::Tensor> bias);
+at::Tensor gelu_fwd(at::Tensor pre, c10::optional<at::Tensor> bias, bool tanh_form);
+std::tuple<at::Tensor, at::Tensor> gelu_bwd(at::Tensor dact, at::Tensor pre, c10::optional<at::Tensor> bias, bool tanh_form,
+                                            c10::optional<at::Tensor> dbias_out);
 std::tuple<at::Tensor, at::Tensor> eden_compress(at::Tensor x, at::Tensor levels, int64_t bits, int64_t seed, int64_t step);
 at::Tensor eden_decompress(at::Tensor words, at::Tensor scale, at::Tensor levels, int64_t n, int64_t bits, int64_t seed,
                            int64_t step);
@@ -102,6 +105,8 @@ TORCH_LIBRARY(dq, m) {
         "Tensor(a!)? dw_out=None, Tensor(b!)? db_out=None, Tensor(c!)? dbias_out=None) -> (Tensor, Tensor, Tensor, Tensor)",
         &dq::add_norm_bwd);
   m.def("residual_add(Tensor x, Tensor delta, Tensor? bias) -> Tensor", &dq::residual_add);
+  m.def("gelu_fwd(Tensor pre, Tensor? bias, bool tanh_form) -> Tensor", &dq::gelu_fwd);
+  m.def("gelu_bwd(Tensor dact, Tensor pre, Tensor? bias, bool tanh_form, Tensor(a!)? dbias_out=None) -> (Tensor, Tensor)", &dq::gelu_bwd);
   m.def("eden_compress(Tensor x, Tensor levels, int bits, int seed, int step) -> (Tensor, Tensor)", &dq::eden_compress);
   m.def("eden_decompress(Tensor words, Tensor scale, Tensor levels, int n, int bits, int seed, int step) -> Tensor",
         &dq::eden_decompress);
