@@ -62,6 +62,10 @@ at::Tensor residual_add(at::Tensor x, at::Tensor delta, c10::optional<at::Tensor
 at::Tensor gelu_fwd(at::Tensor pre, c10::optional<at::Tensor> bias, bool tanh_form);
 std::tuple<at::Tensor, at::Tensor> gelu_bwd(at::Tensor dact, at::Tensor pre, c10::optional<at::Tensor> bias, bool tanh_form,
                                             c10::optional<at::Tensor> dbias_out);
+void rope_qkv_(at::Tensor qkv, at::Tensor cos, at::Tensor sin, int64_t nh, int64_t nkv, int64_t D);
+std::tuple<at::Tensor, at::Tensor> qkv_grad_pack(at::Tensor dq, at::Tensor dk, at::Tensor dv, c10::optional<at::Tensor> cos,
+                                                 c10::optional<at::Tensor> sin, bool want_bias,
+                                                 c10::optional<at::Tensor> dbias_out);
 std::tuple<at::Tensor, at::Tensor> eden_compress(at::Tensor x, at::Tensor levels, int64_t bits, int64_t seed, int64_t step);
 at::Tensor eden_decompress(at::Tensor words, at::Tensor scale, at::Tensor levels, int64_t n, int64_t bits, int64_t seed,
                            int64_t step);
@@ -107,6 +111,9 @@ TORCH_LIBRARY(dq, m) {
   m.def("residual_add(Tensor x, Tensor delta, Tensor? bias) -> Tensor", &dq::residual_add);
   m.def("gelu_fwd(Tensor pre, Tensor? bias, bool tanh_form) -> Tensor", &dq::gelu_fwd);
   m.def("gelu_bwd(Tensor dact, Tensor pre, Tensor? bias, bool tanh_form, Tensor(a!)? dbias_out=None) -> (Tensor, Tensor)", &dq::gelu_bwd);
+  m.def("rope_qkv_(Tensor(a!) qkv, Tensor cos, Tensor sin, int nh, int nkv, int D) -> ()", &dq::rope_qkv_);
+  m.def("qkv_grad_pack(Tensor dq, Tensor dk, Tensor dv, Tensor? cos, Tensor? sin, bool want_bias, Tensor(a!)? dbias_out=None) -> "
+        "(Tensor, Tensor)", &dq::qkv_grad_pack);
   m.def("eden_compress(Tensor x, Tensor levels, int bits, int seed, int step) -> (Tensor, Tensor)", &dq::eden_compress);
   m.def("eden_decompress(Tensor words, Tensor scale, Tensor levels, int n, int bits, int seed, int step) -> Tensor",
         &dq::eden_decompress);
