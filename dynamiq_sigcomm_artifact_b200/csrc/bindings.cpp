@@ -66,6 +66,8 @@ void rope_qkv_(at::Tensor qkv, at::Tensor cos, at::Tensor sin, int64_t nh, int64
 std::tuple<at::Tensor, at::Tensor> qkv_grad_pack(at::Tensor dq, at::Tensor dk, at::Tensor dv, c10::optional<at::Tensor> cos,
                                                  c10::optional<at::Tensor> sin, bool want_bias,
                                                  c10::optional<at::Tensor> dbias_out);
+at::Tensor embed_fwd(at::Tensor ids, at::Tensor tok, c10::optional<at::Tensor> pos, c10::optional<at::Tensor> typ);
+void embed_bwd(at::Tensor dx, at::Tensor ids, c10::optional<at::Tensor> tok_grad, c10::optional<at::Tensor> pos_grad);
 std::tuple<at::Tensor, at::Tensor> eden_compress(at::Tensor x, at::Tensor levels, int64_t bits, int64_t seed, int64_t step);
 at::Tensor eden_decompress(at::Tensor words, at::Tensor scale, at::Tensor levels, int64_t n, int64_t bits, int64_t seed,
                            int64_t step);
@@ -114,6 +116,8 @@ TORCH_LIBRARY(dq, m) {
   m.def("rope_qkv_(Tensor(a!) qkv, Tensor cos, Tensor sin, int nh, int nkv, int D) -> ()", &dq::rope_qkv_);
   m.def("qkv_grad_pack(Tensor dq, Tensor dk, Tensor dv, Tensor? cos, Tensor? sin, bool want_bias, Tensor(a!)? dbias_out=None) -> "
         "(Tensor, Tensor)", &dq::qkv_grad_pack);
+  m.def("embed_fwd(Tensor ids, Tensor tok, Tensor? pos, Tensor? typ) -> Tensor", &dq::embed_fwd);
+  m.def("embed_bwd(Tensor dx, Tensor ids, Tensor(a!)? tok_grad, Tensor(b!)? pos_grad) -> ()", &dq::embed_bwd);
   m.def("eden_compress(Tensor x, Tensor levels, int bits, int seed, int step) -> (Tensor, Tensor)", &dq::eden_compress);
   m.def("eden_decompress(Tensor words, Tensor scale, Tensor levels, int n, int bits, int seed, int step) -> Tensor",
         &dq::eden_decompress);
