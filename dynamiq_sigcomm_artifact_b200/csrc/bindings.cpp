@@ -68,6 +68,10 @@ std::tuple<at::Tensor, at::Tensor> qkv_grad_pack(at::Tensor dq, at::Tensor dk, a
                                                  c10::optional<at::Tensor> dbias_out);
 at::Tensor embed_fwd(at::Tensor ids, at::Tensor tok, c10::optional<at::Tensor> pos, c10::optional<at::Tensor> typ);
 void embed_bwd(at::Tensor dx, at::Tensor ids, c10::optional<at::Tensor> tok_grad, c10::optional<at::Tensor> pos_grad);
+bool ce_fused_fits(int64_t stride);
+std::tuple<at::Tensor, at::Tensor> ce_fused(at::Tensor logits, at::Tensor labels, int64_t vocab, int64_t ignore_index, bool shift,
+                                            bool want_colsum);
+void ce_rescale_(at::Tensor grad, at::Tensor g);
 std::tuple<at::Tensor, at::Tensor> eden_compress(at::Tensor x, at::Tensor levels, int64_t bits, int64_t seed, int64_t step);
 at::Tensor eden_decompress(at::Tensor words, at::Tensor scale, at::Tensor levels, int64_t n, int64_t bits, int64_t seed,
                            int64_t step);
@@ -118,6 +122,10 @@ TORCH_LIBRARY(dq, m) {
         "(Tensor, Tensor)", &dq::qkv_grad_pack);
   m.def("embed_fwd(Tensor ids, Tensor tok, Tensor? pos, Tensor? typ) -> Tensor", &dq::embed_fwd);
   m.def("embed_bwd(Tensor dx, Tensor ids, Tensor(a!)? tok_grad, Tensor(b!)? pos_grad) -> ()", &dq::embed_bwd);
+  m.def("ce_fused_fits(int stride) -> bool", &dq::ce_fused_fits);
+  m.def("ce_fused(Tensor(a!) logits, Tensor labels, int vocab, int ignore_index, bool shift, bool colsum) -> (Tensor, Tensor)",
+        &dq::ce_fused);
+  m.def("ce_rescale_(Tensor(a!) grad, Tensor g) -> ()", &dq::ce_rescale_);
   m.def("eden_compress(Tensor x, Tensor levels, int bits, int seed, int step) -> (Tensor, Tensor)", &dq::eden_compress);
   m.def("eden_decompress(Tensor words, Tensor scale, Tensor levels, int n, int bits, int seed, int step) -> Tensor",
         &dq::eden_decompress);
