@@ -9,7 +9,8 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops.embedding import TiedEmbedding
-from ..ops.layers import LayerNorm, fused_cross_entropy, padded_vocab_logits, shift_labels
+from ..ops.blocks import add_norm
+from ..ops.layers import LayerNorm
 from ..ops.linear import MasterLinear
 from .common import GeluMLP, SelfAttention, init_linear
 
@@ -42,9 +43,18 @@ class BertLayer(nn.Module):
         self.ln1, self.ln2 = LayerNorm(c.hidden, c.eps), LayerNorm(c.hidden, c.eps)
         self.mlp = GeluMLP(c.hidden, c.intermediate, approximate="none")
 
-    def forward(self, x):
-        x = self.ln1(x + self.attn(x))
-        return self.ln2(x + self.mlp(x))
+    def fusable(self, x) -> bool:
+        return self.attn.fusable(x) and self.mlp.fusable(x)
+
+    def forward(self, x, res=None):
+        """`res`: x once more, for the residual addition; then the result comes twice as well, so that backward gets
+        the two gradients apart and adds them inside the norm's pass."""
+        if not self.fusable(x):
+            x = self.ln1(x + self.attn(x))
+            return self.ln2(x + self.mlp(x))
+        h, h_res = add_norm(self.ln1, x if res is None else res, self.attn(x, with_bias=False), self.attn.proj.bias, post=True)
+        y, y_res = add_norm(self.ln2, h_res, self.mlp(h, with_bias=False), self.mlp.proj.bias, post=True)
+        return y if res is None else (y, y_res)
 
 
 class BertMLM(nn.Module):
@@ -59,22 +69,29 @@ class BertMLM(nn.Module):
         self.head_dense = MasterLinear(c.hidden, c.hidden)
         self.head_ln = LayerNorm(c.hidden, c.eps)
         self.head_bias = nn.Parameter(torch.zeros(c.vocab))
+        self.chain_blocks = True  # False: layers are called one by one (their graphs take and return one tensor)
         self.apply(init_linear)
 
     def forward(self, input_ids: torch.Tensor, labels: torch.Tensor | None = None):
         B, S = input_ids.shape
-        pos = torch.arange(S, device=input_ids.device)
-        x = self.tok(input_ids) + self.pos(pos) + self.typ.weight[0]
-        if torch.is_autocast_enabled(x.device.type):
-            x = x.to(torch.get_autocast_dtype(x.device.type))
-        x = self.ln_emb(x)
-        for layer in self.layers:
-            x = layer(x)
+        x = self.tok.embed(input_ids, self.pos.weight, self.typ.weight) if S <= self.config.max_pos else None
+        if x is None:
+            pos = torch.arange(S, device=input_ids.device)
+            x = self.tok(input_ids) + self.pos(pos) + self.typ.weight[0]
+            if torch.is_autocast_enabled(x.device.type):
+                x = x.to(torch.get_autocast_dtype(x.device.type))
+        if self.chain_blocks and len(self.layers) > 0 and self.layers[0].fusable(x):
+            x, res = add_norm(self.ln_emb, x, post=True)
+            for layer in self.layers:
+                x, res = layer(x, res)
+        else:
+            x = self.ln_emb(x)
+            for layer in self.layers:
+                x = layer(x)
         h = self.head_ln(F.gelu(self.head_dense(x)))
         if labels is None:
             return F.linear(h, self.tok.weight.to(h.dtype), self.head_bias.to(h.dtype))
-        logits = self.tok.logits(h, self.head_bias)
-        return fused_cross_entropy(logits, labels.reshape(-1), self.config.vocab)
+        return self.tok.loss(h, labels, self.head_bias)
 
 
 def mask_tokens(input_ids: torch.Tensor, vocab: int, mask_token_id: int, generator: torch.Generator | None = None,

@@ -15,6 +15,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops import blocks
 from ..ops.layers import apply_rope, swiglu
 from ..ops.linear import MasterLinear
 
@@ -40,7 +41,14 @@ class SelfAttention(nn.Module):
         self.qkv = MasterLinear(hidden, (self.n_heads + 2 * self.n_kv) * self.head_dim, bias=bias)
         self.proj = MasterLinear(hidden, hidden, bias=bias)
 
-    def forward(self, x: torch.Tensor, cos=None, sin=None) -> torch.Tensor:
+    def fusable(self, x: torch.Tensor) -> bool:
+        return blocks.fusable(x, self.qkv, self.proj) and self.head_dim % 16 == 0 and not (self.rope and self.qkv.bias is not None)
+
+    def forward(self, x: torch.Tensor, cos=None, sin=None, with_bias: bool = True) -> torch.Tensor:
+        """`with_bias` False (fusable inputs only): the output projection's bias is left to the caller."""
+        if self.fusable(x):
+            return blocks.attention(x, self.qkv, self.proj, self.n_heads, self.n_kv, self.causal, cos if self.rope else None,
+                                    sin if self.rope else None, with_bias)
         B, S, _ = x.shape
         qkv = self.qkv(x)
         q, k, v = qkv.split([self.n_heads * self.head_dim, self.n_kv * self.head_dim, self.n_kv * self.head_dim], -1)
@@ -61,7 +69,13 @@ class GeluMLP(nn.Module):
         self.proj = MasterLinear(inner, hidden)
         self.approximate = approximate
 
-    def forward(self, x):
+    def fusable(self, x: torch.Tensor) -> bool:
+        return blocks.fusable(x, self.fc, self.proj)
+
+    def forward(self, x, with_bias: bool = True):
+        """`with_bias` False (fusable inputs only): the output projection's bias is left to the caller."""
+        if self.fusable(x):
+            return blocks.mlp(x, self.fc, self.proj, self.approximate == "tanh", with_bias)
         return self.proj(F.gelu(self.fc(x), approximate=self.approximate))
 
 

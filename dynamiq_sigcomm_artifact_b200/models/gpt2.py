@@ -9,7 +9,8 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops.embedding import TiedEmbedding
-from ..ops.layers import LayerNorm, fused_cross_entropy, shift_labels
+from ..ops.blocks import add_norm, residual_add
+from ..ops.layers import LayerNorm
 from .common import GeluMLP, SelfAttention, init_linear
 
 
@@ -35,9 +36,20 @@ class GPT2Block(nn.Module):
         self.attn = SelfAttention(c.d_model, c.n_head, causal=True)
         self.mlp = GeluMLP(c.d_model, c.d_mlp)
 
-    def forward(self, x):
-        x = x + self.attn(self.ln1(x))
-        return x + self.mlp(self.ln2(x))
+    def fusable(self, x) -> bool:
+        return self.attn.fusable(x) and self.mlp.fusable(x)
+
+    def forward(self, x, delta=None, delta_bias=None, chained: bool = False):
+        """`chained`: x, delta and delta_bias are what the previous block returned (the first block gets x alone), and
+        the result is (residual stream, this block's last contribution, its bias) for the next block to add up."""
+        if not self.fusable(x):
+            x = x + self.attn(self.ln1(x))
+            return x + self.mlp(self.ln2(x))
+        x, h = add_norm(self.ln1, x, delta, delta_bias)
+        a = self.attn(h, with_bias=False)
+        x, h = add_norm(self.ln2, x, a, self.attn.proj.bias)
+        m = self.mlp(h, with_bias=False)
+        return (x, m, self.mlp.proj.bias) if chained else residual_add(x, m, self.mlp.proj.bias)
 
 
 class GPT2(nn.Module):
@@ -48,6 +60,7 @@ class GPT2(nn.Module):
         self.wpe = nn.Embedding(c.context, c.d_model)
         self.blocks = nn.ModuleList(GPT2Block(c) for _ in range(c.n_layer))
         self.ln_f = LayerNorm(c.d_model, c.eps)
+        self.chain_blocks = True  # False: blocks are called one by one (their graphs take and return one tensor)
         self.apply(init_linear)
         for b in self.blocks:  # GPT-2's scaled init of the residual projections
             nn.init.normal_(b.attn.proj.weight, std=0.02 / (2 * c.n_layer) ** 0.5)
@@ -55,14 +68,21 @@ class GPT2(nn.Module):
 
     def forward(self, input_ids: torch.Tensor, labels: torch.Tensor | None = None):
         B, S = input_ids.shape
-        pos = torch.arange(S, device=input_ids.device)
-        x = self.wte(input_ids) + self.wpe(pos)
-        if torch.is_autocast_enabled(x.device.type):
-            x = x.to(torch.get_autocast_dtype(x.device.type))
-        for blk in self.blocks:
-            x = blk(x)
-        h = self.ln_f(x)
+        x = self.wte.embed(input_ids, self.wpe.weight) if S <= self.config.context else None
+        if x is None:
+            pos = torch.arange(S, device=input_ids.device)
+            x = self.wte(input_ids) + self.wpe(pos)
+            if torch.is_autocast_enabled(x.device.type):
+                x = x.to(torch.get_autocast_dtype(x.device.type))
+        if self.chain_blocks and len(self.blocks) > 0 and self.blocks[0].fusable(x):
+            delta = bias = None
+            for blk in self.blocks:
+                x, delta, bias = blk(x, delta, bias, True)
+            h = add_norm(self.ln_f, x, delta, bias)[1]
+        else:
+            for blk in self.blocks:
+                x = blk(x)
+            h = self.ln_f(x)
         if labels is None:
             return F.linear(h, self.wte.weight)
-        logits = self.wte.logits(h)
-        return fused_cross_entropy(logits, shift_labels(labels).reshape(-1), self.config.vocab)
+        return self.wte.loss(h, labels, shift=True)

@@ -9,6 +9,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops.embedding import TiedEmbedding
+from ..ops.blocks import add_norm, residual_add
 from ..ops.layers import fused_cross_entropy, padded_vocab_logits, shift_labels, RMSNorm, rope_tables
 from .common import SelfAttention, SwiGLU, init_linear
 
@@ -38,9 +39,18 @@ class LlamaBlock(nn.Module):
         self.attn = SelfAttention(c.d_model, c.n_head, c.n_kv_head, bias=False, causal=True, rope=True)
         self.mlp = SwiGLU(c.d_model, c.d_ffn)
 
-    def forward(self, x, cos, sin):
-        x = x + self.attn(self.norm1(x), cos, sin)
-        return x + self.mlp(self.norm2(x))
+    def fusable(self, x) -> bool:
+        return self.attn.fusable(x)
+
+    def forward(self, x, cos, sin, delta=None, chained: bool = False):
+        """`chained`: x and delta are what the previous block returned (the first block gets x alone), and the result is
+        (residual stream, this block's last contribution) for the next block to add up."""
+        if not self.fusable(x):
+            x = x + self.attn(self.norm1(x), cos, sin)
+            return x + self.mlp(self.norm2(x))
+        x, h = add_norm(self.norm1, x, delta)
+        x, h = add_norm(self.norm2, x, self.attn(h, cos, sin))
+        return (x, self.mlp(h)) if chained else residual_add(x, self.mlp(h))
 
 
 class Llama(nn.Module):
@@ -51,6 +61,7 @@ class Llama(nn.Module):
         self.blocks = nn.ModuleList(LlamaBlock(c) for _ in range(c.n_layer))
         self.norm = RMSNorm(c.d_model, c.eps)
         self.lm_head = None if c.tie_embeddings else nn.Linear(c.d_model, c.vocab, bias=False)
+        self.chain_blocks = True  # False: blocks are called one by one (their graphs take and return one tensor)
         self.apply(init_linear)
         self._rope = None
 
@@ -63,14 +74,23 @@ class Llama(nn.Module):
     def forward(self, input_ids: torch.Tensor, labels: torch.Tensor | None = None):
         B, S = input_ids.shape
         cos, sin = self._tables(S, input_ids.device)
-        x = self.embed(input_ids)
-        if torch.is_autocast_enabled(x.device.type):
-            x = x.to(torch.get_autocast_dtype(x.device.type))
-        for blk in self.blocks:
-            x = blk(x, cos, sin)
+        x = self.embed.embed(input_ids)
+        if x is None:
+            x = self.embed(input_ids)
+            if torch.is_autocast_enabled(x.device.type):
+                x = x.to(torch.get_autocast_dtype(x.device.type))
+        if self.chain_blocks and len(self.blocks) > 0 and self.blocks[0].fusable(x):
+            delta = None
+            for blk in self.blocks:
+                x, delta = blk(x, cos, sin, delta, True)
+            h = add_norm(self.norm, x, delta)[1]
+        else:
+            for blk in self.blocks:
+                x = blk(x, cos, sin)
+            h = self.norm(x)
         w = self.embed.weight if self.lm_head is None else self.lm_head.weight
-        h = self.norm(x)
         if labels is None:
             return F.linear(h, w)
-        logits = self.embed.logits(h) if self.lm_head is None else padded_vocab_logits(h, w)
-        return fused_cross_entropy(logits, shift_labels(labels).reshape(-1), self.config.vocab)
+        if self.lm_head is None:
+            return self.embed.loss(h, labels, shift=True)
+        return fused_cross_entropy(padded_vocab_logits(h, w), shift_labels(labels).reshape(-1), self.config.vocab)

@@ -22,6 +22,9 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import require
+from ..utils import counters
+
 PAD_ROWS = 128
 
 
@@ -73,6 +76,75 @@ class _HeadFn(torch.autograd.Function):
         return dh, dw, None
 
 
+class _EmbedFn(torch.autograd.Function):
+    """bf16(token row + position row [+ type row 0]) in one kernel; see csrc/kernels/embedding_ops.cu."""
+
+    @staticmethod
+    def forward(ctx, ids, weight, shadow, pos, typ):
+        ctx.save_for_backward(ids)
+        ctx.shapes = (weight.shape, None if pos is None else pos.shape, None if typ is None else typ.shape)
+        ctx.direct = getattr(weight, "_dq_grad_padded", None)
+        ctx.sparse = getattr(weight, "_dq_sparse", None)
+        counters.add("embed_fwd")
+        return require().embed_fwd(ids, shadow, pos, typ)
+
+    @staticmethod
+    def backward(ctx, dx):
+        (ids,) = ctx.saved_tensors
+        tok, pos, typ = ctx.shapes
+        dx = dx.contiguous()
+        dw = None
+        if ctx.sparse is not None:
+            ctx.sparse["ids"], ctx.sparse["rows"] = ids.reshape(-1), dx.view(-1, dx.shape[-1])
+            target = None
+        elif ctx.direct is not None:
+            target = ctx.direct  # holds the output projection's weight gradient, written earlier in this backward pass
+        else:
+            target = dw = torch.zeros(tok, dtype=torch.float32, device=dx.device)
+        dpos = None if pos is None else torch.empty(pos, dtype=torch.float32, device=dx.device)
+        if target is not None or dpos is not None:
+            require().embed_bwd(dx, ids, target, dpos)
+            counters.add("embed_bwd")
+        dtyp = None
+        if typ is not None:
+            dtyp = torch.zeros(typ, dtype=torch.float32, device=dx.device)
+            require().colsum(dx.view(-1, dx.shape[-1]), dtyp[0])
+            counters.add("colsum", 2)
+        return None, dw, None, dpos, dtyp
+
+
+class _HeadLossFn(torch.autograd.Function):
+    """Mean cross-entropy of h W^T (+ bias) with the gradient of the logits written over them in the same pass
+    (csrc/kernels/loss_fused.cu): the logits exist only between this node's two halves."""
+
+    @staticmethod
+    def forward(ctx, h, weight, shadow, bias, low_bias, labels, vocab: int, ignore_index: int, shift: bool):
+        h2 = h.reshape(-1, h.shape[-1])
+        logits = F.linear(h2, shadow, low_bias)
+        loss, sums = require().ce_fused(logits, labels.contiguous(), vocab, ignore_index, shift, bias is not None)
+        counters.add("ce_fused", 3 if bias is None else 4)
+        ctx.save_for_backward(h, shadow, logits, sums)
+        ctx.rows, ctx.has_bias = weight.shape[0], bias is not None
+        ctx.direct = getattr(weight, "_dq_grad_padded", None)
+        return loss
+
+    @staticmethod
+    def backward(ctx, g):
+        h, shadow, dlogits, sums = ctx.saved_tensors
+        g = g.to(torch.float32).reshape(1)
+        require().ce_rescale_(dlogits, g)
+        counters.add("ce_rescale")
+        h2 = h.reshape(-1, h.shape[-1])
+        dh = (dlogits @ shadow).view(h.shape) if ctx.needs_input_grad[0] else None
+        dw = None
+        if ctx.direct is not None:
+            torch.mm(dlogits.t(), h2, out_dtype=torch.float32, out=ctx.direct)  # overwrites: first contribution
+        else:
+            dw = torch.mm(dlogits.t(), h2, out_dtype=torch.float32)[: ctx.rows]
+        db = sums[: ctx.rows] * g if ctx.has_bias else None
+        return dh, dw, None, db, None, None, None, None, None
+
+
 class TiedEmbedding(nn.Embedding):
     """``nn.Embedding`` whose weight also serves as the output projection.
 
@@ -108,6 +180,31 @@ class TiedEmbedding(nn.Embedding):
 
     def forward(self, ids: torch.Tensor) -> torch.Tensor:
         return self.lookup(ids)
+
+    def embed(self, ids: torch.Tensor, pos: Optional[torch.Tensor] = None, typ: Optional[torch.Tensor] = None
+              ) -> Optional[torch.Tensor]:
+        """bf16 rows of `ids` [B, S] plus the first S rows of `pos` plus row 0 of `typ`, or None where the fused kernel
+        does not apply (no bf16 working copy in use)."""
+        if not self._use_shadow(ids.device.type) or self.embedding_dim % 8 != 0 or ids.dim() != 2 or ids.dtype != torch.int64:
+            return None
+        return _EmbedFn.apply(ids.contiguous(), self.weight, self.shadow, pos, typ)
+
+    def loss(self, h: torch.Tensor, labels: torch.Tensor, bias: Optional[torch.Tensor] = None, shift: bool = False,
+             ignore_index: int = -100) -> torch.Tensor:
+        """Mean cross-entropy of ``logits(h, bias)`` against `labels` [B, S]; `shift`: position t predicts t + 1."""
+        from .layers import fused_cross_entropy, shift_labels
+
+        fused = self._use_shadow(h.device.type) and h.dtype == torch.bfloat16 and torch.is_grad_enabled() \
+            and h.requires_grad and labels.dtype == torch.int64 and require().ce_fused_fits(self.padded_rows)
+        if not fused:
+            if shift:
+                labels = shift_labels(labels)
+            return fused_cross_entropy(self.logits(h, bias), labels.reshape(-1), self.num_embeddings, ignore_index)
+        low = None
+        if bias is not None:
+            low = torch.zeros(self.padded_rows, dtype=torch.bfloat16, device=h.device)
+            low[: self.num_embeddings].copy_(bias.detach())
+        return _HeadLossFn.apply(h, self.weight, self.shadow, bias, low, labels, self.num_embeddings, ignore_index, shift)
 
     def logits(self, h: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
         if self._use_shadow(h.device.type) and h.dtype == torch.bfloat16:

@@ -15,9 +15,12 @@ import torch.nn.functional as F
 
 from . import require
 from ..utils import counters
+from .blocks import add_norm
 
 
 class _NormFn(torch.autograd.Function):
+    """Hidden sizes beyond those of blocks.add_norm (2048)."""
+
     @staticmethod
     def forward(ctx, x, w, b, eps: float, rms: bool):
         ops = require()
@@ -58,6 +61,8 @@ class LayerNorm(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if x.is_cuda:
+            if x.shape[-1] <= 2048:
+                return add_norm(self, x)[1]
             return _NormFn.apply(x, self.weight.float(), self.bias.float(), self.eps, False)
         return F.layer_norm(x.float(), (x.shape[-1],), self.weight.float(), self.bias.float(), self.eps).to(x.dtype)
 
@@ -70,6 +75,8 @@ class RMSNorm(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if x.is_cuda:
+            if x.shape[-1] <= 2048:
+                return add_norm(self, x)[1]
             return _NormFn.apply(x, self.weight.float(), None, self.eps, True)
         xf = x.float()
         return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps) * self.weight.float()).to(x.dtype)

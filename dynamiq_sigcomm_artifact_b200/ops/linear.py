@@ -24,12 +24,12 @@ class _ShadowLinearFn(torch.autograd.Function):
     ``None`` (no temporary, no accumulate kernel).  In that mode a backward pass overwrites."""
 
     @staticmethod
-    def forward(ctx, x, weight, shadow, bias):
+    def forward(ctx, x, weight, shadow, bias, low_bias):
         ctx.save_for_backward(x, shadow)
         ctx.has_bias = bias is not None
         ctx.wg = getattr(weight, "_dq_grad", None)
         ctx.bg = getattr(bias, "_dq_grad", None) if bias is not None else None
-        return F.linear(x, shadow, None if bias is None else bias.to(x.dtype))
+        return F.linear(x, shadow, low_bias)
 
     @staticmethod
     def backward(ctx, dy):
@@ -55,7 +55,7 @@ class _ShadowLinearFn(torch.autograd.Function):
                 db = dy2.sum(dim=0, dtype=torch.float32)
             if ctx.bg is not None:
                 db = None
-        return dx, dw, None, db
+        return dx, dw, None, db, None
 
 
 class MasterLinear(nn.Module):
@@ -67,7 +67,14 @@ class MasterLinear(nn.Module):
         self.weight = nn.Parameter(torch.empty(out_features, in_features))
         self.bias = nn.Parameter(torch.zeros(out_features)) if bias else None
         nn.init.kaiming_uniform_(self.weight, a=math.sqrt(5))
-        self.shadow = None  # bf16 copy, created by enable_shadows()
+        self.shadow = None  # bf16 copies of weight and bias, created by enable_shadows()
+        self.bias_shadow = None
+
+    def low_bias(self):
+        """The bias as the bf16 GEMMs take it."""
+        if self.bias is None:
+            return None
+        return self.bias_shadow if self.bias_shadow is not None else self.bias.detach().to(torch.bfloat16)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if self.shadow is not None and x.is_cuda:
@@ -75,12 +82,13 @@ class MasterLinear(nn.Module):
                     and torch.get_autocast_dtype("cuda") == torch.bfloat16:
                 x = x.to(torch.bfloat16)
             if x.dtype == torch.bfloat16:
-                return _ShadowLinearFn.apply(x, self.weight, self.shadow, self.bias)
+                return _ShadowLinearFn.apply(x, self.weight, self.shadow, self.bias, self.low_bias())
         return F.linear(x, self.weight, self.bias)
 
 
 def enable_shadows(model: nn.Module) -> Dict[nn.Parameter, torch.Tensor]:
-    """Create (or refresh) the bf16 copy of every MasterLinear / TiedEmbedding weight; returns {weight: copy}
+    """Create (or refresh) the bf16 copies of every MasterLinear's weight and bias and every TiedEmbedding's weight;
+    returns {parameter: copy}
     (a TiedEmbedding's copy has extra zero rows after the parameter's)."""
     from .embedding import TiedEmbedding
 
@@ -94,4 +102,10 @@ def enable_shadows(model: nn.Module) -> Dict[nn.Parameter, torch.Tensor]:
             with torch.no_grad():
                 m.shadow.copy_(m.weight)
             out[m.weight] = m.shadow
+            if m.bias is not None:
+                if m.bias_shadow is None or m.bias_shadow.device != m.bias.device:
+                    m.bias_shadow = torch.empty_like(m.bias, dtype=torch.bfloat16)
+                with torch.no_grad():
+                    m.bias_shadow.copy_(m.bias)
+                out[m.bias] = m.bias_shadow
     return out

@@ -212,6 +212,7 @@ class Trainer:
         blocks = getattr(m, "blocks", None) or getattr(m, "layers", None)
         if blocks is None:
             return False
+        m.chain_blocks = False
         c = m.config
         hidden = getattr(c, "d_model", None) or getattr(c, "hidden")
         x = torch.randn(cfg.micro_batch, cfg.seq_len, hidden, device=self.device, dtype=torch.bfloat16,
@@ -241,6 +242,7 @@ class Trainer:
         except Exception as e:  # fall back to eager execution, loudly
             print(f"[dynamiq] CUDA graph capture of the blocks failed ({type(e).__name__}: {e}); running eagerly",
                   flush=True)
+            m.chain_blocks = True
             return False
         for i, g in enumerate(graphed):
             blocks[i] = g
