@@ -15,10 +15,16 @@ struct SharedDivisor {
   float b, r;
   __device__ __forceinline__ explicit SharedDivisor(float divisor) : b(divisor), r(1.0f / divisor) {}
 
-  __device__ __forceinline__ float operator()(float a) const {
+  // the caller knows that the numerator, the divisor and the quotient are within 1e-20 .. 1e20 or does not mind an
+  // error of a few units in a quotient below (its sign is right, and zero comes out as zero)
+  __device__ __forceinline__ float in_range(float a) const {
     float q = __fmul_rn(a, r);
     q = __fmaf_rn(__fmaf_rn(-b, q, a), r, q);
-    q = __fmaf_rn(__fmaf_rn(-b, q, a), r, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, a), r, q);
+  }
+
+  __device__ __forceinline__ float operator()(float a) const {
+    float q = in_range(a);
     const float m = fabsf(q), n = fabsf(a);
     if (!(m >= 1e-20f && m <= 1e20f && n >= 1e-20f && n <= 1e20f)) q = a == 0.0f ? a : __fdiv_rn(a, b);
     return q;

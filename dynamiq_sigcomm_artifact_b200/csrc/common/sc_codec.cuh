@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "exact_div.cuh"
 #include "philox.cuh"
 #include "rht_codec.cuh"
 
@@ -109,6 +110,185 @@ __device__ __forceinline__ void sc_store_block_coalesced(float* base, float* buf
   __syncwarp();
 }
 
+// ---- a lane's two chunks as one byte stream ----
+// A lane's part of a record is [codes of chunk 0][scale][codes of chunk 1][scale]: 4 b + 2 bytes (34 / 18 / 10) at an even
+// offset.  It is put together in registers and moved with 32-bit shared-memory accesses (two 16-bit ones where the offset
+// is not a multiple of four), instead of byte by byte.
+
+// `B` codes per byte stream of a chunk: four bytes-of-codes words (code 4 j + i in byte i of c[j]) -> B / 2 words
+template <int B>
+__device__ __forceinline__ void sc_pack16(const uint32_t (&c)[4], uint32_t (&w)[B / 2 > 0 ? B / 2 : 1]) {
+  if constexpr (B == 8) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = c[j];
+  } else if constexpr (B == 4) {
+    uint32_t t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) t[j] = c[j] | (c[j] >> 4);  // bytes 0 and 2 hold two codes each
+    w[0] = __byte_perm(t[0], t[1], 0x6420u);
+    w[1] = __byte_perm(t[2], t[3], 0x6420u);
+  } else {
+    uint32_t t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t p = c[j] | (c[j] >> 6);  // bytes 0 and 2 hold two codes each
+      t[j] = p | (p >> 12);                   // byte 0 holds four
+    }
+    w[0] = __byte_perm(__byte_perm(t[0], t[1], 0x0040u), __byte_perm(t[2], t[3], 0x0040u), 0x5410u);
+  }
+}
+
+template <int B>
+__device__ __forceinline__ void sc_unpack16(const uint32_t (&w)[B / 2 > 0 ? B / 2 : 1], uint32_t (&c)[4]) {
+  if constexpr (B == 8) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[j] = w[j];
+  } else if constexpr (B == 4) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t t = __byte_perm(w[j >> 1], 0u, (j & 1) ? 0x4342u : 0x4140u);  // two bytes into bytes 0 and 2
+      c[j] = (t | (t << 4)) & 0x0F0F0F0Fu;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t t = __byte_perm(w[0], 0u, 0x4440u + j);
+      const uint32_t p = (t | (t << 12)) & 0x000F000Fu;
+      c[j] = (p | (p << 6)) & 0x03030303u;
+    }
+  }
+}
+
+// codes of both chunks (as bytes) and their scale bytes -> the lane's stream at `dst` (shared memory, even address)
+template <int B>
+__device__ __forceinline__ void sc_put_stream(uint8_t* dst, const uint32_t (&c0)[4], const uint32_t (&c1)[4], uint32_t q0,
+                                              uint32_t q1) {
+  constexpr int W = B / 2;  // code words per chunk: 1, 2, 4
+  uint32_t a[W], b[W], w[2 * W + 2];
+  sc_pack16<B>(c0, a);
+  sc_pack16<B>(c1, b);
+#pragma unroll
+  for (int j = 0; j < W; ++j) w[j] = a[j];
+  w[W] = q0 | (b[0] << 8);
+#pragma unroll
+  for (int j = 1; j < W; ++j) w[W + j] = __funnelshift_l(b[j - 1], b[j], 8);
+  w[2 * W] = (b[W - 1] >> 24) | (q1 << 8);  // 16 bits
+  w[2 * W + 1] = 0u;
+  const uint32_t odd = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(dst)) & 2u;
+  if (odd) *reinterpret_cast<uint16_t*>(dst) = static_cast<uint16_t>(w[0]);
+  uint32_t* at = reinterpret_cast<uint32_t*>(dst + odd);
+#pragma unroll
+  for (int j = 0; j < 2 * W; ++j) at[j] = __funnelshift_r(w[j], w[j + 1], 8 * odd);
+  if (!odd) *reinterpret_cast<uint16_t*>(at + 2 * W) = static_cast<uint16_t>(w[2 * W]);
+}
+
+template <int B>
+__device__ __forceinline__ void sc_get_stream(const uint8_t* src, uint32_t (&c0)[4], uint32_t (&c1)[4], uint32_t& q0,
+                                              uint32_t& q1) {
+  constexpr int W = B / 2;
+  uint32_t r[2 * W + 1], w[2 * W + 1], a[W], b[W];
+  const uint32_t odd = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(src)) & 2u;
+  const uint32_t* at = reinterpret_cast<const uint32_t*>(src - odd);  // the last word may reach two bytes past the stream:
+#pragma unroll                                                       // inside the tile, whose size is a multiple of four
+  for (int j = 0; j < 2 * W + 1; ++j) r[j] = at[j];
+#pragma unroll
+  for (int j = 0; j < 2 * W; ++j) w[j] = __funnelshift_r(r[j], r[j + 1], 8 * odd);
+  w[2 * W] = odd ? r[2 * W] >> 16 : r[2 * W];
+#pragma unroll
+  for (int j = 0; j < W; ++j) a[j] = w[j];
+  q0 = w[W] & 0xFFu;
+#pragma unroll
+  for (int j = 0; j < W; ++j) b[j] = __funnelshift_r(w[W + j], w[W + j + 1], 8);
+  q1 = (w[2 * W] >> 8) & 0xFFu;
+  sc_unpack16<B>(a, c0);
+  sc_unpack16<B>(b, c1);
+}
+
+// ---- one lane's 32 values <-> codes (bytes, four per word) and chunk scales ----
+// The record's arithmetic with every division done through SharedDivisor: the divisors (chunk scale, lattice constants)
+// are shared by 16 values or by all.  A quotient below 1e-20 only has to keep its sign (it ends as level 0 or -1 + 1
+// either way), so the general division is needed only where a magnitude exceeds 1e20: the whole warp then takes it.
+template <bool MEE>
+__device__ __forceinline__ void sc_encode_lane(const float (&v)[32], float lattice_max, float c1, float c2, int R,
+                                               uint32_t first_call, uint32_t tag, uint32_t step, uint32_t k0, uint32_t k1,
+                                               int lane, uint32_t (&code)[2][4], uint32_t (&scale)[2],
+                                               __nv_bfloat16& unit_bf) {
+  float x[32], am[2], s[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    am[h] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      x[16 * h + k] = sc_sanitize(v[16 * h + k]);
+      am[h] = fmaxf(am[h], fabsf(x[16 * h + k]));
+    }
+    s[h] = fmaxf(__fadd_rn(__fdiv_rn(am[h], lattice_max), 1e-7f), 1e-30f);
+  }
+  float S = fmaxf(s[0], s[1]);
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) S = fmaxf(S, __shfl_xor_sync(0xFFFFFFFFu, S, o));
+  unit_bf = __float2bfloat16_rn(fmaxf(__fdiv_rn(S, 255.0f), 1e-30f));
+  const float unit = fmaxf(__bfloat162float(unit_bf), 1e-30f);
+  const bool wide = __any_sync(0xFFFFFFFFu, S > 1e19f);
+  const SharedDivisor by_c1(c1), by_c2(c2);
+  const float fR = static_cast<float>(R);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float q = fminf(fmaxf(ceilf(__fmul_rn(__fdiv_rn(s[h], S), 255.0f)), 1.0f), 255.0f);
+    const float dec = fmaxf(__fmul_rn(q, unit), 1e-30f);
+    scale[h] = static_cast<uint32_t>(q);
+    float* y = x + 16 * h;
+    if (wide) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) y[k] = __fdiv_rn(y[k], dec);
+    } else {
+      const SharedDivisor by_dec(dec);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) y[k] = by_dec.in_range(y[k]);
+    }
+    const U4 r = philox4x32<7>(first_call + 2u * static_cast<uint32_t>(lane) + h, 0u, tag, step, k0, k1);
+    const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+    uint32_t f[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      float t = y[k];
+      if (MEE) {
+        const float mag = by_c2.in_range(log2f(__fadd_rn(by_c1.in_range(fabsf(t)), 1.0f)));
+        t = t > 0.f ? mag : (t < 0.f ? -mag : 0.f);
+      }
+      // 2^15 + byte + 0.5 from one byte permute, then (byte + 0.5) / 256: every step exact
+      const float u = fmaf(__uint_as_float(__byte_perm(rw[k >> 2], 0x47000080u, 0x7504u | ((k & 3) << 4))), 1.0f / 256.0f, -128.0f);
+      const float fl = floorf(t);
+      const float c = fl + ((__fsub_rn(t, fl) > u) ? 1.0f : 0.0f);
+      f[k] = __float_as_uint(__fadd_rn(fminf(fmaxf(c, -fR), fR), 12582912.0f + fR));  // low byte = c + R
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      code[h][j] = __byte_perm(__byte_perm(f[4 * j], f[4 * j + 1], 0x0040u), __byte_perm(f[4 * j + 2], f[4 * j + 3], 0x0040u), 0x5410u);
+  }
+}
+
+// `lut`: decode levels in shared memory (MEE)
+template <bool MEE, bool ADD>
+__device__ __forceinline__ void sc_decode_lane(float (&v)[32], const uint32_t (&code)[2][4], const uint32_t (&scale)[2],
+                                               float unit, const float* lut, int R) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float dec = fmaxf(__fmul_rn(static_cast<float>(scale[h]), unit), 1e-30f);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const uint32_t c = (code[h][k >> 2] >> (8 * (k & 3))) & 0xFFu;
+      const float level = MEE ? lut[c] : static_cast<float>(static_cast<int>(c) - R);
+      const float val = __fmul_rn(level, dec);
+      v[16 * h + k] = ADD ? __fadd_rn(v[16 * h + k], val) : val;
+    }
+  }
+}
+
+__device__ __forceinline__ float sc_unit_at(const uint8_t* p) {  // p is even
+  return fmaxf(__bfloat162float(__ushort_as_bfloat16(*reinterpret_cast<const unsigned short*>(p))), 1e-30f);
+}
+
 // Encode the block held in v into four records in `tile` (shared memory, >= kBlockBytes).
 template <int B, bool MEE>
 __device__ __forceinline__ void sc_encode_block(const float (&v)[32], uint8_t* tile, const ScParams& sp,
@@ -116,59 +296,13 @@ __device__ __forceinline__ void sc_encode_block(const float (&v)[32], uint8_t* t
                                                 uint32_t k1, int lane) {
   constexpr int R = (1 << (B - 1)) - 1;
   using G = ScGeom<B>;
-  float x[32], s[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    float am = 0.f;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      x[16 * h + k] = sc_sanitize(v[16 * h + k]);
-      am = fmaxf(am, fabsf(x[16 * h + k]));
-    }
-    s[h] = fmaxf(__fadd_rn(__fdiv_rn(am, sp.lattice_max), 1e-7f), 1e-30f);
-  }
-  float S = fmaxf(s[0], s[1]);
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) S = fmaxf(S, __shfl_xor_sync(0xFFFFFFFFu, S, o));
-  const __nv_bfloat16 unit_bf = __float2bfloat16_rn(fmaxf(__fdiv_rn(S, 255.0f), 1e-30f));
-  const float unit = fmaxf(__bfloat162float(unit_bf), 1e-30f);
+  uint32_t code[2][4], scale[2];
+  __nv_bfloat16 unit;
+  sc_encode_lane<MEE>(v, sp.lattice_max, MEE ? sp.c1 : 1.0f, MEE ? sp.c2 : 1.0f, R, first_call, tag, step, k0, k1, lane, code,
+                      scale, unit);
   uint8_t* rec = tile + (lane >> 3) * G::kRecordBytes;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const float q = fminf(fmaxf(ceilf(__fmul_rn(__fdiv_rn(s[h], S), 255.0f)), 1.0f), 255.0f);
-    const float dec = fmaxf(__fmul_rn(q, unit), 1e-30f);
-    U4 r = philox4x32<7>(first_call + 2u * static_cast<uint32_t>(lane) + h, 0u, tag, step, k0, k1);
-    const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
-    uint32_t code[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      float y = __fdiv_rn(x[16 * h + k], dec);
-      if (MEE) {
-        const float mag = __fdiv_rn(log2f(__fadd_rn(__fdiv_rn(fabsf(y), sp.c1), 1.0f)), sp.c2);
-        y = y > 0.f ? mag : (y < 0.f ? -mag : 0.f);
-      }
-      const float u = __fmul_rn(__fadd_rn(static_cast<float>((rw[k >> 2] >> (8 * (k & 3))) & 0xFFu), 0.5f), 1.0f / 256.0f);
-      const float fl = floorf(y);
-      float c = fl + ((__fsub_rn(y, fl) > u) ? 1.0f : 0.0f);
-      c = fminf(fmaxf(c, static_cast<float>(-R)), static_cast<float>(R));
-      code[k] = static_cast<uint32_t>(static_cast<int>(c) + R);
-    }
-    uint8_t* ch = rec + (2 * (lane & 7) + h) * G::kChunkBytes;
-    constexpr int per = 8 / B;  // codes per byte, little end first
-#pragma unroll
-    for (int byte = 0; byte < 2 * B; ++byte) {
-      uint32_t val = 0;
-#pragma unroll
-      for (int j = 0; j < per; ++j) val |= code[byte * per + j] << (j * B);
-      ch[byte] = static_cast<uint8_t>(val);
-    }
-    ch[2 * B] = static_cast<uint8_t>(q);
-  }
-  if ((lane & 7) == 0) {
-    const unsigned short bits = __bfloat16_as_ushort(unit_bf);
-    rec[16 * G::kChunkBytes] = static_cast<uint8_t>(bits & 0xFF);
-    rec[16 * G::kChunkBytes + 1] = static_cast<uint8_t>(bits >> 8);
-  }
+  sc_put_stream<B>(rec + 2 * (lane & 7) * G::kChunkBytes, code[0], code[1], scale[0], scale[1]);
+  if ((lane & 7) == 0) *reinterpret_cast<__nv_bfloat16*>(rec + 16 * G::kChunkBytes) = unit;
 }
 
 // Decode the four records in `tile`; ADD: v <- v + decoded (one rounding each), else v <- decoded.
@@ -177,22 +311,9 @@ __device__ __forceinline__ void sc_decode_block(float (&v)[32], const uint8_t* t
   constexpr int R = (1 << (B - 1)) - 1;
   using G = ScGeom<B>;
   const uint8_t* rec = tile + (lane >> 3) * G::kRecordBytes;
-  const unsigned short ub = static_cast<unsigned short>(rec[16 * G::kChunkBytes]) |
-                            (static_cast<unsigned short>(rec[16 * G::kChunkBytes + 1]) << 8);
-  const float unit = fmaxf(__bfloat162float(__ushort_as_bfloat16(ub)), 1e-30f);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const uint8_t* ch = rec + (2 * (lane & 7) + h) * G::kChunkBytes;
-    const float dec = fmaxf(__fmul_rn(static_cast<float>(ch[2 * B]), unit), 1e-30f);
-    constexpr int per = 8 / B;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const uint32_t code = (static_cast<uint32_t>(ch[k / per]) >> ((k % per) * B)) & ((1u << B) - 1u);
-      const float level = MEE ? sp.lut[code] : static_cast<float>(static_cast<int>(code) - R);
-      const float val = __fmul_rn(level, dec);
-      v[16 * h + k] = ADD ? __fadd_rn(v[16 * h + k], val) : val;
-    }
-  }
+  uint32_t code[2][4], scale[2];
+  sc_get_stream<B>(rec + 2 * (lane & 7) * G::kChunkBytes, code[0], code[1], scale[0], scale[1]);
+  sc_decode_lane<MEE, ADD>(v, code, scale, sc_unit_at(rec + 16 * G::kChunkBytes), sp.lut, R);
 }
 
 // shared-memory tile <-> global record area, 8 bytes per lane per trip
@@ -237,65 +358,24 @@ __device__ __forceinline__ int sc_mix_rec_base(uint32_t wpack, int g) {
   return base;
 }
 
+// `table` is the constant table, in shared memory
 template <bool MEE>
 __device__ __forceinline__ void sc_encode_block_mix(const float (&v)[32], uint8_t* tile, const float* table,
                                                     uint32_t wpack, uint32_t first_call, uint32_t tag, uint32_t step,
                                                     uint32_t k0, uint32_t k1, int lane) {
   const int g = lane >> 3;
   const int B = static_cast<int>((wpack >> (8 * g)) & 0xFF);
-  const int R = (1 << (B - 1)) - 1;
-  const int ti = sc_mix_slot(B);
-  const float lattice_max = __ldg(table + ti), c1 = __ldg(table + 4 + ti), c2 = __ldg(table + 8 + ti);
-  const int chunk_bytes = 2 * B + 1;
-  float x[32], s[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    float am = 0.f;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      x[16 * h + k] = sc_sanitize(v[16 * h + k]);
-      am = fmaxf(am, fabsf(x[16 * h + k]));
-    }
-    s[h] = fmaxf(__fadd_rn(__fdiv_rn(am, lattice_max), 1e-7f), 1e-30f);
-  }
-  float S = fmaxf(s[0], s[1]);
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) S = fmaxf(S, __shfl_xor_sync(0xFFFFFFFFu, S, o));
-  const __nv_bfloat16 unit_bf = __float2bfloat16_rn(fmaxf(__fdiv_rn(S, 255.0f), 1e-30f));
-  const float unit = fmaxf(__bfloat162float(unit_bf), 1e-30f);
+  const int ti = sc_mix_slot(B), chunk_bytes = 2 * B + 1;
+  uint32_t code[2][4], scale[2];
+  __nv_bfloat16 unit;
+  sc_encode_lane<MEE>(v, table[ti], MEE ? table[4 + ti] : 1.0f, MEE ? table[8 + ti] : 1.0f, (1 << (B - 1)) - 1, first_call,
+                      tag, step, k0, k1, lane, code, scale, unit);
   uint8_t* rec = tile + sc_mix_rec_base(wpack, g);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const float q = fminf(fmaxf(ceilf(__fmul_rn(__fdiv_rn(s[h], S), 255.0f)), 1.0f), 255.0f);
-    const float dec = fmaxf(__fmul_rn(q, unit), 1e-30f);
-    U4 r = philox4x32<7>(first_call + 2u * static_cast<uint32_t>(lane) + h, 0u, tag, step, k0, k1);
-    const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
-    unsigned long long acc[2] = {0ull, 0ull};
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      float y = __fdiv_rn(x[16 * h + k], dec);
-      if (MEE) {
-        const float mag = __fdiv_rn(log2f(__fadd_rn(__fdiv_rn(fabsf(y), c1), 1.0f)), c2);
-        y = y > 0.f ? mag : (y < 0.f ? -mag : 0.f);
-      }
-      const float u = __fmul_rn(__fadd_rn(static_cast<float>((rw[k >> 2] >> (8 * (k & 3))) & 0xFFu), 0.5f), 1.0f / 256.0f);
-      const float fl = floorf(y);
-      float c = fl + ((__fsub_rn(y, fl) > u) ? 1.0f : 0.0f);
-      c = fminf(fmaxf(c, static_cast<float>(-R)), static_cast<float>(R));
-      acc[k >> 3] |= static_cast<unsigned long long>(static_cast<uint32_t>(static_cast<int>(c) + R)) << ((k & 7) * B);
-    }
-    uint8_t* ch = rec + (2 * (lane & 7) + h) * chunk_bytes;
-    for (int byte = 0; byte < B; ++byte) {  // codes 0..7 fill B bytes, codes 8..15 the next B, little end first
-      ch[byte] = static_cast<uint8_t>(acc[0] >> (8 * byte));
-      ch[B + byte] = static_cast<uint8_t>(acc[1] >> (8 * byte));
-    }
-    ch[2 * B] = static_cast<uint8_t>(q);
-  }
-  if ((lane & 7) == 0) {
-    const unsigned short bits = __bfloat16_as_ushort(unit_bf);
-    rec[16 * chunk_bytes] = static_cast<uint8_t>(bits & 0xFF);
-    rec[16 * chunk_bytes + 1] = static_cast<uint8_t>(bits >> 8);
-  }
+  uint8_t* at = rec + 2 * (lane & 7) * chunk_bytes;
+  if (B == 8) sc_put_stream<8>(at, code[0], code[1], scale[0], scale[1]);
+  else if (B == 4) sc_put_stream<4>(at, code[0], code[1], scale[0], scale[1]);
+  else sc_put_stream<2>(at, code[0], code[1], scale[0], scale[1]);
+  if ((lane & 7) == 0) *reinterpret_cast<__nv_bfloat16*>(rec + 16 * chunk_bytes) = unit;
 }
 
 template <bool MEE, bool ADD>
@@ -303,31 +383,14 @@ __device__ __forceinline__ void sc_decode_block_mix(float (&v)[32], const uint8_
                                                     uint32_t wpack, int lane) {
   const int g = lane >> 3;
   const int B = static_cast<int>((wpack >> (8 * g)) & 0xFF);
-  const int R = (1 << (B - 1)) - 1;
-  const uint32_t mask = (1u << B) - 1u;
   const int chunk_bytes = 2 * B + 1;
-  const float* lut = table + sc_mix_lut_base(B);
   const uint8_t* rec = tile + sc_mix_rec_base(wpack, g);
-  const unsigned short ub = static_cast<unsigned short>(rec[16 * chunk_bytes]) |
-                            (static_cast<unsigned short>(rec[16 * chunk_bytes + 1]) << 8);
-  const float unit = fmaxf(__bfloat162float(__ushort_as_bfloat16(ub)), 1e-30f);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const uint8_t* ch = rec + (2 * (lane & 7) + h) * chunk_bytes;
-    const float dec = fmaxf(__fmul_rn(static_cast<float>(ch[2 * B]), unit), 1e-30f);
-    unsigned long long acc[2] = {0ull, 0ull};
-    for (int byte = 0; byte < B; ++byte) {
-      acc[0] |= static_cast<unsigned long long>(ch[byte]) << (8 * byte);
-      acc[1] |= static_cast<unsigned long long>(ch[B + byte]) << (8 * byte);
-    }
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const uint32_t code = static_cast<uint32_t>(acc[k >> 3] >> ((k & 7) * B)) & mask;
-      const float level = MEE ? __ldg(lut + code) : static_cast<float>(static_cast<int>(code) - R);
-      const float val = __fmul_rn(level, dec);
-      v[16 * h + k] = ADD ? __fadd_rn(v[16 * h + k], val) : val;
-    }
-  }
+  const uint8_t* at = rec + 2 * (lane & 7) * chunk_bytes;
+  uint32_t code[2][4], scale[2];
+  if (B == 8) sc_get_stream<8>(at, code[0], code[1], scale[0], scale[1]);
+  else if (B == 4) sc_get_stream<4>(at, code[0], code[1], scale[0], scale[1]);
+  else sc_get_stream<2>(at, code[0], code[1], scale[0], scale[1]);
+  sc_decode_lane<MEE, ADD>(v, code, scale, sc_unit_at(rec + 16 * chunk_bytes), table + sc_mix_lut_base(B), (1 << (B - 1)) - 1);
 }
 
 __device__ __forceinline__ void sc_copy_out_n(uint8_t* dst, const uint8_t* tile, int n8, int lane) {

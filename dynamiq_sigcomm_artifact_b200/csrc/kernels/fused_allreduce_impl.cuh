@@ -78,6 +78,10 @@ __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
   if (!SC) fill_sign_tables(sgn_fwd, sgn_inv, sign_words, p.finish_scale, tid, blockDim.x);
+  // the superchunk codecs keep their constants and decode levels where the rotation codec has its sign table
+  const float* levels = sgn_fwd;
+  if (MIX || CODEC == kCodecScMee)
+    for (int i = tid; i < (MIX ? kScMixTableFloats : 1 << SCB); i += blockDim.x) sgn_fwd[i] = p.sc_lut[i];
   __syncthreads();
 
   T* bucket = static_cast<T*>(p.bucket);
@@ -94,7 +98,7 @@ __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
   // the rotation codec and the identity wire read raw blocks in the coalesced load layout, which a bulk copy into
   // the warp's staging buffer can prefetch; the other record codecs use that buffer to form lane-contiguous runs
   bool prefetch_ok = (!SC || CAST) && use_stage;
-  const ScParams scp{p.sc_lattice_max, p.sc_c1, p.sc_c2, p.sc_lut};
+  const ScParams scp{p.sc_lattice_max, p.sc_c1, p.sc_c2, levels};
   uint8_t* rec_tile = reinterpret_cast<uint8_t*>(tile);  // superchunk codec: the warp's record staging area
   auto issue_prefetch = [&](RawItem it) {
     pf = RawItem{-1, -1};
@@ -193,7 +197,7 @@ __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
           else sc_copy_out<SCB>(dstp, rec_tile, lane);
         };
         auto rec_encode = [&]() {
-          if constexpr (MIX) sc_encode_block_mix<MEE>(v, rec_tile, p.sc_lut, wpack, first_call, tag, p.step, p.seed_lo, p.seed_hi, lane);
+          if constexpr (MIX) sc_encode_block_mix<MEE>(v, rec_tile, levels, wpack, first_call, tag, p.step, p.seed_lo, p.seed_hi, lane);
           else if constexpr (CAST) cast_encode_block<CB>(v, rec_tile, lane);
           else if constexpr (MX) mx_encode_block<MXB>(v, rec_tile, lane);
           else sc_encode_block<SCB, MEE>(v, rec_tile, scp, first_call, tag, p.step, p.seed_lo, p.seed_hi, lane);
@@ -273,7 +277,7 @@ __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
             for (int r = 0; r < nrecv; ++r) {
               const uint8_t* slot = my_mail + static_cast<unsigned long long>(recv_slot + r) * p.slot_stride;
               rec_in(slot + boff);
-              if constexpr (MIX) sc_decode_block_mix<MEE, true>(v, rec_tile, p.sc_lut, wpack, lane);
+              if constexpr (MIX) sc_decode_block_mix<MEE, true>(v, rec_tile, levels, wpack, lane);
               else if constexpr (CAST) cast_decode_block<CB, true>(v, rec_tile, lane);
               else if constexpr (MX) mx_decode_block<MXB, true>(v, rec_tile, lane);
               else sc_decode_block<SCB, MEE, true>(v, rec_tile, scp, lane);
@@ -299,7 +303,7 @@ __device__ __forceinline__ void fused_simt_body(const ARParams& p) {
             } else {
               rec_in(my_mail + static_cast<unsigned long long>(recv_slot) * p.slot_stride + boff);
             }
-            if constexpr (MIX) sc_decode_block_mix<MEE, false>(v, rec_tile, p.sc_lut, wpack, lane);
+            if constexpr (MIX) sc_decode_block_mix<MEE, false>(v, rec_tile, levels, wpack, lane);
             else if constexpr (CAST) cast_decode_block<CB, false>(v, rec_tile, lane);
             else if constexpr (MX) mx_decode_block<MXB, false>(v, rec_tile, lane);
             else sc_decode_block<SCB, MEE, false>(v, rec_tile, scp, lane);
