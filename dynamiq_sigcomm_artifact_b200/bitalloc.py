@@ -137,8 +137,8 @@ class DeviceBitrateController:
 
     ``state`` is four doubles on the device (u, initialised, last average width, last delta).  Every
     bucket's widths come from ``torch.ops.dq.superchunk_widths`` (which also returns the scores it
-    used); after the step's last bucket the scores are sorted once and one small kernel walks the
-    bisection / adjustment with binary searches (csrc/kernels/bitalloc_ops.cu).  The update runs on the
+    used); after the step's last bucket one small kernel walks the bisection / adjustment, counting over
+    the scores (csrc/kernels/bitalloc_ops.cu).  The update runs on the
     stream it is called on and is published through ``ready`` (an event) for the next step's first bucket.
     Widths come from thresholds on the score (8 from 8 up, 4 from 4 up, else 2), which is
     :func:`qbits` without the round trip through ``log2``.
@@ -172,7 +172,7 @@ class DeviceBitrateController:
             return
         s = torch.cat(self._scores) if len(self._scores) > 1 else self._scores[0]
         self._scores = []
-        _ops.require().superchunk_bitrate_update(torch.sort(s).values, self.state, self.target)
+        _ops.require().superchunk_bitrate_update(s, self.state, self.target)
         self.ready = torch.cuda.Event()
         self.ready.record(torch.cuda.current_stream(self.device))
 

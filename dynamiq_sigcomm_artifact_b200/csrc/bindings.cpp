@@ -78,7 +78,7 @@ at::Tensor eden_decompress(at::Tensor words, at::Tensor scale, at::Tensor levels
 at::Tensor fwht_pow2(at::Tensor x, double scale, bool clean);
 void superchunk_widths(at::Tensor stats, at::Tensor state, at::Tensor s_out, at::Tensor widths);
 at::Tensor superchunk_plan(at::Tensor widths);
-void superchunk_bitrate_update(at::Tensor sorted_s, at::Tensor state, double target);
+void superchunk_bitrate_update(at::Tensor scores, at::Tensor state, double target);
 void nvls_allreduce(at::Tensor bucket, int64_t stage_ptr, int64_t mc_ptr, std::vector<int64_t> flag_ptrs,
                     int64_t stage_bytes, int64_t status_ptr, int64_t rank, int64_t world, int64_t wire_bits, int64_t epoch,
                     double post_scale, int64_t timeout_ns, int64_t ctas);
@@ -132,7 +132,7 @@ TORCH_LIBRARY(dq, m) {
   m.def("fwht_pow2(Tensor x, float scale, bool clean) -> Tensor", &dq::fwht_pow2);
   m.def("superchunk_widths(Tensor stats, Tensor state, Tensor(a!) s_out, Tensor(b!) widths) -> ()", &dq::superchunk_widths);
   m.def("superchunk_plan(Tensor widths) -> Tensor", &dq::superchunk_plan);
-  m.def("superchunk_bitrate_update(Tensor sorted_s, Tensor(a!) state, float target) -> ()", &dq::superchunk_bitrate_update);
+  m.def("superchunk_bitrate_update(Tensor scores, Tensor(a!) state, float target) -> ()", &dq::superchunk_bitrate_update);
   m.def("rht_widths_update(Tensor mailbox, Tensor(a!) plan, int nblocks, int blocks_per_shard, int slot_stride, "
         "int scales_off, int first_ag_slot, int budget) -> ()", &dq::rht_widths_update);
   m.def("nvls_allreduce(Tensor(a!) bucket, int stage_ptr, int mc_ptr, int[] flag_ptrs, int stage_bytes, int status_ptr, "

@@ -53,11 +53,27 @@ __global__ void __launch_bounds__(256) sc_center_kernel(const T* __restrict__ x,
   }
 }
 
+// four values and one mean per thread and step, two steps in flight (one value at a time: 12.8 us for 25 MB, 0.63 of the
+// copy rate); out is 4-element aligned where this runs, the residual always is
+__global__ void __launch_bounds__(256) sc_add_mean_vec_kernel(const float* __restrict__ resid, const float* __restrict__ mean,
+                                                              float* __restrict__ out, long long n4) {
+  const long long step = gridDim.x * 256ll;
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n4; i += 2 * step) {
+    const long long j = i + step;
+    const float4 a = __ldcs(reinterpret_cast<const float4*>(resid) + i);
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (j < n4) b = __ldcs(reinterpret_cast<const float4*>(resid) + j);
+    const float ma = mean[i >> 6], mb = j < n4 ? mean[j >> 6] : 0.f;
+    reinterpret_cast<float4*>(out)[i] = make_float4(a.x + ma, a.y + ma, a.z + ma, a.w + ma);
+    if (j < n4) reinterpret_cast<float4*>(out)[j] = make_float4(b.x + mb, b.y + mb, b.z + mb, b.w + mb);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) sc_add_mean_kernel(const float* __restrict__ resid,
                                                           const float* __restrict__ mean, T* __restrict__ out,
-                                                          long long n) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
+                                                          long long first, long long n) {
+  for (long long i = first + blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x)
     st_from_float(out, i, resid[i] + mean[i >> 8]);
 }
@@ -93,12 +109,22 @@ void superchunk_add_mean(at::Tensor resid, at::Tensor mean, at::Tensor out) {
   TORCH_CHECK(resid.numel() >= n && mean.numel() * 256 >= n, "superchunk_add_mean: residual / mean too short");
   if (n == 0) return;
   c10::cuda::CUDAGuard guard(out.device());
-  const int grid = static_cast<int>(std::min<long long>((n + 255) / 256, 148LL * 16));
+  long long done = 0;
   auto stream = at::cuda::getCurrentCUDAStream();
+  if (out.scalar_type() == at::kFloat &&
+      ((reinterpret_cast<uintptr_t>(out.data_ptr()) | reinterpret_cast<uintptr_t>(resid.data_ptr())) & 15u) == 0 && n >= 4) {
+    const long long n4 = n / 4;
+    sc_add_mean_vec_kernel<<<static_cast<int>(std::min<long long>((n4 + 511) / 512, 148LL * 8)), 256, 0, stream>>>(
+        resid.data_ptr<float>(), mean.data_ptr<float>(), out.data_ptr<float>(), n4);
+    C10_CUDA_KERNEL_LAUNCH_CHECK();
+    done = 4 * n4;
+    if (done == n) return;
+  }
+  const int grid = static_cast<int>(std::min<long long>((n - done + 255) / 256, 148LL * 16));
   if (out.scalar_type() == at::kFloat)
-    sc_add_mean_kernel<float><<<grid, 256, 0, stream>>>(resid.data_ptr<float>(), mean.data_ptr<float>(), out.data_ptr<float>(), n);
+    sc_add_mean_kernel<float><<<grid, 256, 0, stream>>>(resid.data_ptr<float>(), mean.data_ptr<float>(), out.data_ptr<float>(), done, n);
   else if (out.scalar_type() == at::kBFloat16)
-    sc_add_mean_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(resid.data_ptr<float>(), mean.data_ptr<float>(), reinterpret_cast<__nv_bfloat16*>(out.data_ptr()), n);
+    sc_add_mean_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(resid.data_ptr<float>(), mean.data_ptr<float>(), reinterpret_cast<__nv_bfloat16*>(out.data_ptr()), done, n);
   else
     TORCH_CHECK(false, "superchunk_add_mean: fp32 or bf16 output");
   C10_CUDA_KERNEL_LAUNCH_CHECK();

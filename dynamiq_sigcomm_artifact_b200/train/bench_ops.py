@@ -109,8 +109,7 @@ def main(argv=None) -> None:
     widths = torch.empty(nsc, dtype=torch.uint8, device=dev)
     timed("superchunk_widths_256Ki", lambda: dq.superchunk_widths(stats, state, scores, widths), nsc * 13)
     timed("superchunk_plan_256Ki", lambda: dq.superchunk_plan(widths), nsc * 3)
-    sorted_scores = torch.sort(scores).values
-    timed("superchunk_bitrate_update_256Ki", lambda: dq.superchunk_bitrate_update(sorted_scores, state, 4.375), nsc * 4)
+    timed("superchunk_bitrate_update_256Ki", lambda: dq.superchunk_bitrate_update(scores, state, 4.375), nsc * 4)
     # Walsh-Hadamard transform of a whole THC partition: two passes over the vector
     v = torch.randn(1 << 23, device=dev)
     from ..ops.fwht import fwht_pow2
