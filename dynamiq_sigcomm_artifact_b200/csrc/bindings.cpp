@@ -57,15 +57,15 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_fwd(at::Tens
 std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_bwd(
     at::Tensor dy, c10::optional<at::Tensor> dy2, c10::optional<at::Tensor> ds, at::Tensor s, at::Tensor w, at::Tensor mean,
     at::Tensor rstd, bool rms, bool want_bias, c10::optional<at::Tensor> dw_out, c10::optional<at::Tensor> db_out,
-    c10::optional<at::Tensor> dbias_out, int64_t sum_stream);
+    c10::optional<at::Tensor> dbias_out);
 at::Tensor residual_add(at::Tensor x, at::Tensor delta, c10::optional<at::Tensor> bias);
 at::Tensor gelu_fwd(at::Tensor pre, c10::optional<at::Tensor> bias, bool tanh_form);
 std::tuple<at::Tensor, at::Tensor> gelu_bwd(at::Tensor dact, at::Tensor pre, c10::optional<at::Tensor> bias, bool tanh_form,
-                                            c10::optional<at::Tensor> dbias_out, int64_t sum_stream);
+                                            c10::optional<at::Tensor> dbias_out);
 void rope_qkv_(at::Tensor qkv, at::Tensor cos, at::Tensor sin, int64_t nh, int64_t nkv, int64_t D);
 std::tuple<at::Tensor, at::Tensor> qkv_grad_pack(at::Tensor dq, at::Tensor dk, at::Tensor dv, c10::optional<at::Tensor> cos,
                                                  c10::optional<at::Tensor> sin, bool want_bias,
-                                                 c10::optional<at::Tensor> dbias_out, int64_t sum_stream);
+                                                 c10::optional<at::Tensor> dbias_out);
 at::Tensor embed_fwd(at::Tensor ids, at::Tensor tok, c10::optional<at::Tensor> pos, c10::optional<at::Tensor> typ);
 void embed_bwd(at::Tensor dx, at::Tensor ids, c10::optional<at::Tensor> tok_grad, c10::optional<at::Tensor> pos_grad);
 bool ce_fused_fits(int64_t stride);
@@ -112,13 +112,13 @@ TORCH_LIBRARY(dq, m) {
   m.def("add_norm_fwd(Tensor x, Tensor? delta, Tensor? bias, Tensor w, Tensor? b, float eps, bool rms) -> (Tensor, Tensor, Tensor, Tensor)",
         &dq::add_norm_fwd);
   m.def("add_norm_bwd(Tensor dy, Tensor? dy2, Tensor? ds, Tensor s, Tensor w, Tensor mean, Tensor rstd, bool rms, bool want_bias, "
-        "Tensor(a!)? dw_out=None, Tensor(b!)? db_out=None, Tensor(c!)? dbias_out=None, int sum_stream=0) -> (Tensor, Tensor, Tensor, Tensor)",
+        "Tensor(a!)? dw_out=None, Tensor(b!)? db_out=None, Tensor(c!)? dbias_out=None) -> (Tensor, Tensor, Tensor, Tensor)",
         &dq::add_norm_bwd);
   m.def("residual_add(Tensor x, Tensor delta, Tensor? bias) -> Tensor", &dq::residual_add);
   m.def("gelu_fwd(Tensor pre, Tensor? bias, bool tanh_form) -> Tensor", &dq::gelu_fwd);
-  m.def("gelu_bwd(Tensor dact, Tensor pre, Tensor? bias, bool tanh_form, Tensor(a!)? dbias_out=None, int sum_stream=0) -> (Tensor, Tensor)", &dq::gelu_bwd);
+  m.def("gelu_bwd(Tensor dact, Tensor pre, Tensor? bias, bool tanh_form, Tensor(a!)? dbias_out=None) -> (Tensor, Tensor)", &dq::gelu_bwd);
   m.def("rope_qkv_(Tensor(a!) qkv, Tensor cos, Tensor sin, int nh, int nkv, int D) -> ()", &dq::rope_qkv_);
-  m.def("qkv_grad_pack(Tensor dq, Tensor dk, Tensor dv, Tensor? cos, Tensor? sin, bool want_bias, Tensor(a!)? dbias_out=None, int sum_stream=0) -> "
+  m.def("qkv_grad_pack(Tensor dq, Tensor dk, Tensor dv, Tensor? cos, Tensor? sin, bool want_bias, Tensor(a!)? dbias_out=None) -> "
         "(Tensor, Tensor)", &dq::qkv_grad_pack);
   m.def("embed_fwd(Tensor ids, Tensor tok, Tensor? pos, Tensor? typ) -> Tensor", &dq::embed_fwd);
   m.def("embed_bwd(Tensor dx, Tensor ids, Tensor(a!)? tok_grad, Tensor(b!)? pos_grad) -> ()", &dq::embed_bwd);

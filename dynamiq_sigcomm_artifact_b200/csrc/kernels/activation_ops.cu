@@ -11,8 +11,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include "column_sums.cuh"
 #include "norm_kernels.cuh"
-#include "sum_stream.cuh"
 
 namespace dq {
 namespace {
@@ -194,7 +194,7 @@ at::Tensor gelu_fwd(at::Tensor pre, c10::optional<at::Tensor> bias, bool tanh_fo
 
 // (dpre, dbias); dbias is empty without a bias, and written to dbias_out when that is given
 std::tuple<at::Tensor, at::Tensor> gelu_bwd(at::Tensor dact, at::Tensor pre, c10::optional<at::Tensor> bias, bool tanh_form,
-                                            c10::optional<at::Tensor> dbias_out, int64_t sum_stream) {
+                                            c10::optional<at::Tensor> dbias_out) {
   check_act(pre, bias);
   check_act(dact, bias);
   TORCH_CHECK(dact.scalar_type() == pre.scalar_type() && dact.numel() == pre.numel(), "gelu_bwd: gradient and input must agree");
@@ -224,7 +224,10 @@ std::tuple<at::Tensor, at::Tensor> gelu_bwd(at::Tensor dact, at::Tensor pre, c10
   }
 #undef DQ_CALL
   C10_CUDA_KERNEL_LAUNCH_CHECK();
-  if (bias.has_value()) finish_sums(part, dbias.data_ptr<float>(), nullptr, nullptr, 1, splits, cols, sum_stream);
+  if (bias.has_value()) {
+    reduce_arrays(pp, dbias.data_ptr<float>(), nullptr, nullptr, 1, splits, cols, stream);
+    C10_CUDA_KERNEL_LAUNCH_CHECK();
+  }
   return {dpre, dbias};
 }
 

@@ -11,8 +11,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include "column_sums.cuh"
 #include "norm_kernels.cuh"
-#include "sum_stream.cuh"
 
 namespace dq {
 namespace {
@@ -185,7 +185,7 @@ void rope_qkv_(at::Tensor qkv, at::Tensor cos, at::Tensor sin, int64_t nh, int64
 // dk; want_bias: fp32 column sums of dqkv (into dbias_out when given), zeros for the key part.  One of the two.
 std::tuple<at::Tensor, at::Tensor> qkv_grad_pack(at::Tensor dq, at::Tensor dk, at::Tensor dv, c10::optional<at::Tensor> cos,
                                                  c10::optional<at::Tensor> sin, bool want_bias,
-                                                 c10::optional<at::Tensor> dbias_out, int64_t sum_stream) {
+                                                 c10::optional<at::Tensor> dbias_out) {
   TORCH_CHECK(dq.dim() == 4 && (dq.scalar_type() == at::kBFloat16 || dq.scalar_type() == at::kFloat), "qkv_grad_pack: bf16 or fp32 [B, heads, S, D]");
   const int64_t B = dq.size(0), nh = dq.size(1), S = dq.size(2), D = dq.size(3), nkv = dk.size(1);
   TORCH_CHECK(D % 8 == 0 && nkv >= 1, "qkv_grad_pack: head dimension must be a multiple of 8");
@@ -226,7 +226,10 @@ std::tuple<at::Tensor, at::Tensor> qkv_grad_pack(at::Tensor dq, at::Tensor dk, a
   if (dq.scalar_type() == at::kBFloat16) DQ_CALL(__nv_bfloat16); else DQ_CALL(float);
 #undef DQ_CALL
   C10_CUDA_KERNEL_LAUNCH_CHECK();
-  if (want_bias) finish_sums(part, dbias.data_ptr<float>(), nullptr, nullptr, 1, splits, static_cast<int>(cols), sum_stream);
+  if (want_bias) {
+    reduce_arrays(part.data_ptr<float>(), dbias.data_ptr<float>(), nullptr, nullptr, 1, splits, static_cast<int>(cols), stream);
+    C10_CUDA_KERNEL_LAUNCH_CHECK();
+  }
   return {out, dbias};
 }
 

@@ -21,7 +21,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_fwd(at::Tens
 std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_bwd(
     at::Tensor dy, c10::optional<at::Tensor> dy2, c10::optional<at::Tensor> ds, at::Tensor s, at::Tensor w, at::Tensor mean,
     at::Tensor rstd, bool rms, bool want_bias, c10::optional<at::Tensor> dw_out, c10::optional<at::Tensor> db_out,
-    c10::optional<at::Tensor> dbias_out, int64_t sum_stream);
+    c10::optional<at::Tensor> dbias_out);
 
 namespace {
 
@@ -381,7 +381,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> norm_bwd(at::Tensor dy, at::Tenso
   c10::cuda::CUDAGuard guard(x.device());
   const int H = static_cast<int>(x.size(-1));
   if (norm_rows_fit(H)) {
-    auto out = add_norm_bwd(dy, c10::nullopt, c10::nullopt, x, w, mean, rstd, rms, false, dw_out, db_out, c10::nullopt, 0);
+    auto out = add_norm_bwd(dy, c10::nullopt, c10::nullopt, x, w, mean, rstd, rms, false, dw_out, db_out, c10::nullopt);
     return {std::get<0>(out), std::get<1>(out), std::get<2>(out)};
   }
   const int rows = static_cast<int>(x.numel() / H);

@@ -17,8 +17,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include "column_sums.cuh"
 #include "norm_kernels.cuh"
-#include "sum_stream.cuh"
 
 namespace dq {
 namespace {
@@ -188,11 +188,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_fwd(at::Tens
 }
 
 // Returns (dx, dw, db, dbias); db is empty for RMSNorm, dbias unless `want_bias`.  dw_out / db_out / dbias_out: where
-// the column sums go instead of new tensors; sum_stream: see sum_stream.cuh.
+// the column sums go instead of new tensors.
 std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_bwd(
     at::Tensor dy, c10::optional<at::Tensor> dy2, c10::optional<at::Tensor> ds, at::Tensor s, at::Tensor w, at::Tensor mean,
     at::Tensor rstd, bool rms, bool want_bias, c10::optional<at::Tensor> dw_out, c10::optional<at::Tensor> db_out,
-    c10::optional<at::Tensor> dbias_out, int64_t sum_stream) {
+    c10::optional<at::Tensor> dbias_out) {
   TORCH_CHECK(s.is_cuda() && s.is_contiguous() && (s.scalar_type() == at::kBFloat16 || s.scalar_type() == at::kFloat),
               "norm_bwd: contiguous bf16 or fp32 CUDA activations");
   const int H = static_cast<int>(s.size(-1));
@@ -231,7 +231,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_bwd(
 #undef DQ_BWD
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   float* second = rms ? (want_bias ? dbias.data_ptr<float>() : nullptr) : db.data_ptr<float>();
-  finish_sums(part, dw.data_ptr<float>(), second, want_bias ? dbias.data_ptr<float>() : nullptr, arrays, grid, H, sum_stream);
+  reduce_arrays(part.data_ptr<float>(), dw.data_ptr<float>(), second, want_bias ? dbias.data_ptr<float>() : nullptr, arrays,
+                grid, H, stream);
+  C10_CUDA_KERNEL_LAUNCH_CHECK();
   return {dx, dw, db, dbias};
 }
 

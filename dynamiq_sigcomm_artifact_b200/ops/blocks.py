@@ -35,19 +35,6 @@ def _arena(p) -> Optional[torch.Tensor]:
     return getattr(p, "_dq_grad", None) if p is not None else None
 
 
-def _sum_stream(*params) -> int:
-    """Handle of the stream that finishes the column sums of these parameters' gradients, 0 for the current one: the
-    bucket reducer's side stream when all of them live in its arena (csrc/kernels/sum_stream.cuh)."""
-    found = 0
-    for p in params:
-        if p is None:
-            continue
-        found = getattr(p, "_dq_sum_stream", 0)
-        if not found:
-            return 0
-    return found
-
-
 def _weight_grad(dy2: torch.Tensor, x2: torch.Tensor, out: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     """dy^T x in fp32, into the arena view when there is one (autograd then sees None)."""
     if out is not None:
@@ -66,7 +53,6 @@ class _AddNormFn(torch.autograd.Function):
         ctx.save_for_backward(s, w, mean, rstd)
         ctx.rms, ctx.post, ctx.has_delta, ctx.has_bias = rms, post, delta is not None, bias is not None and delta is not None
         ctx.wg, ctx.bg, ctx.biasg = _arena(w), _arena(b), _arena(bias)
-        ctx.sums = _sum_stream(w, b, bias if ctx.has_bias else None)
         return (y, y.view_as(y)) if post else (x.view_as(x) if delta is None else s, y)
 
     @staticmethod
@@ -77,7 +63,7 @@ class _AddNormFn(torch.autograd.Function):
             dy, dy2 = (dy2, None) if dy2 is not None else (torch.zeros_like(s), None)
         dx, dw, db, dbias = require().add_norm_bwd(
             dy.contiguous(), None if dy2 is None else dy2.contiguous(), None if ds is None else ds.contiguous(), s, w, mean, rstd,
-            ctx.rms, ctx.has_bias, ctx.wg, ctx.bg, ctx.biasg, ctx.sums)
+            ctx.rms, ctx.has_bias, ctx.wg, ctx.bg, ctx.biasg)
         counters.add("add_norm_bwd", 2)
         return (dx, dx if ctx.has_delta else None, dbias if ctx.has_bias and ctx.biasg is None else None,
                 dw if ctx.wg is None else None, db if not ctx.rms and ctx.bg is None else None, None, None, None)
@@ -123,7 +109,6 @@ class _MlpFn(torch.autograd.Function):
         counters.add("gelu_fwd")
         ctx.save_for_backward(x, pre, act, s1, s2, b1)
         ctx.tanh, ctx.has_b2 = tanh_form, b2 is not None
-        ctx.sums = _sum_stream(b1)
         ctx.arena = (_arena(w1), _arena(b1), _arena(w2), _arena(b2))
         return F.linear(act, s2, b2_low)
 
@@ -134,7 +119,7 @@ class _MlpFn(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         dw2 = _weight_grad(dy2, act.reshape(-1, act.shape[-1]), g2)
         dact = (dy2 @ s2).view_as(pre)
-        dpre, db1 = require().gelu_bwd(dact, pre, b1, ctx.tanh, gb1, ctx.sums)
+        dpre, db1 = require().gelu_bwd(dact, pre, b1, ctx.tanh, gb1)
         counters.add("gelu_bwd", 1 if b1 is None else 2)
         dpre2 = dpre.view(-1, dpre.shape[-1])
         dw1 = _weight_grad(dpre2, x.reshape(-1, x.shape[-1]), g1)
@@ -175,7 +160,6 @@ class _AttentionFn(torch.autograd.Function):
         ctx.save_for_backward(x, o, s1, s2, cos, sin)
         ctx.core, ctx.inputs = (core, (q, k, v)) if grad else (None, None)
         ctx.has_b1, ctx.has_b2 = b1 is not None, b2 is not None
-        ctx.sums = _sum_stream(b1)
         ctx.arena = (_arena(w1), _arena(b1), _arena(w2), _arena(b2))
         return F.linear(o, s2, b2_low)
 
@@ -191,7 +175,7 @@ class _AttentionFn(torch.autograd.Function):
         do = (dy2 @ s2).view(B, S, nh, D).transpose(1, 2)
         dq, dk, dv = (t if t.stride(-1) == 1 else t.contiguous() for t in torch.autograd.grad(core, inputs, do))
         del core, inputs
-        dqkv, db1 = require().qkv_grad_pack(dq, dk, dv, cos, sin, ctx.has_b1, gb1, ctx.sums)
+        dqkv, db1 = require().qkv_grad_pack(dq, dk, dv, cos, sin, ctx.has_b1, gb1)
         counters.add("qkv_grad_pack", 2 if ctx.has_b1 else 1)
         dqkv = dqkv.view(-1, dqkv.shape[-1])
         dw1 = _weight_grad(dqkv, x.reshape(-1, x.shape[-1]), g1)

@@ -138,13 +138,6 @@ class BucketReducer:
         self.groups = self._make_groups(params)
         self._layout(bucket_cap_mb)
         self.side = torch.cuda.Stream(self.device) if (self.cuda and side_stream) else None
-        if self.side is not None and self.world == 1:
-            # column-sum gradients are finished beside backward, in front of their bucket's optimizer step (with several
-            # ranks the blocks are CUDA graphs of their own, which cannot leave work on another stream)
-            for ps in self.bucket_params:
-                for p in ps:
-                    if hasattr(p, "_dq_grad"):
-                        p._dq_sum_stream = self.side.cuda_stream
         self.consumer_stream = torch.cuda.Stream(self.device) if (self.side is not None and self.defer) else None
         self._pending: List[int] = []
         if self.defer:
@@ -279,7 +272,7 @@ class BucketReducer:
         self._handles = []
         for ps in self.bucket_params:
             for p in ps:
-                for a in ("_dq_grad", "_dq_grad_padded", "_dq_sparse", "_dq_sum_stream"):
+                for a in ("_dq_grad", "_dq_grad_padded", "_dq_sparse"):
                     if hasattr(p, a):
                         delattr(p, a)
 
