@@ -52,6 +52,7 @@ void launch_rows(const void* dy, const void* x, const float* w, const float* rst
                  int hidden, int grid, cudaStream_t stream) {
   using namespace dq::normk;
   const int nt = norm_group_threads(hidden);
+  cudaFuncSetAttribute(add_norm_bwd_kernel<T, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNormBwdMaxSmem);
   add_norm_bwd_kernel<T, true, false><<<grid, nt * norm_groups(hidden), norm_bwd_smem(hidden), stream>>>(
       static_cast<const T*>(dy), nullptr, false, static_cast<const T*>(x), w, nullptr, rstd, static_cast<T*>(dx), parts,
       rows, hidden, nt);
@@ -77,8 +78,7 @@ extern "C" int dq_rmsnorm_bwd_noalloc(const void* dy, const void* x, const float
   if (grid > DQ_NOALLOC_MAX_PARTS) grid = DQ_NOALLOC_MAX_PARTS;
   if (is_bf16) launch_rows<__nv_bfloat16>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream);
   else launch_rows<float>(dy, x, w, rstd, dx, parts, rows, hidden, grid, stream);
-  dim3 rb(32, 32);
-  dq::reduce_arrays_kernel<<<(hidden + 31) / 32, rb, 0, stream>>>(parts, dw, nullptr, nullptr, grid, hidden);
+  dq::reduce_arrays(parts, dw, nullptr, nullptr, 1, grid, hidden, stream);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     t_last_cuda_error = static_cast<int>(e);

@@ -95,18 +95,30 @@ struct Raw8<float> {
 // ---- backward of rows with H <= 2048 ----
 // A CTA holds several groups of NT threads (a multiple of 32, at least H / 8), one row per group at a time and eight
 // columns per thread, so that the column sums of dw, db and dbias are 8 registers each; a group synchronises once a row
-// on a barrier of its own, and its next row is already in flight.  At the end the groups add their sums in a fixed order
-// in shared memory and the CTA leaves one partial row: part[arrays][gridDim.x][H], arrays = dw, (db), (dbias).
+// on a barrier of its own.  Every thread brings its own columns of the next rows into its own slots of a shared-memory
+// ring with asynchronous copies (no registers, no barrier).  At the end the groups add their sums in a fixed order in
+// shared memory and the CTA leaves one partial row: part[arrays][gridDim.x][H], arrays = dw, (db), (dbias).
 // `extra` (may be null): a second term of dy, or one of dx.
 constexpr int kNormBwdThreads = 384;  // two CTAs per SM at 80 registers
+template <typename T>
+constexpr int norm_ring() { return sizeof(T) == 2 ? 4 : 2; }  // rows of the ring
 
 inline int norm_group_threads(int H) { return (H / 8 + 31) / 32 * 32; }
 inline int norm_groups(int H) { return kNormBwdThreads / norm_group_threads(H) < 8 ? kNormBwdThreads / norm_group_threads(H) : 8; }
-inline size_t norm_bwd_smem(int H) { return static_cast<size_t>(H) * sizeof(float); }
+// column sums of the groups, then the ring: three tensors x 8 values per thread and row
+inline size_t norm_bwd_smem(int H) {
+  return static_cast<size_t>(H) * sizeof(float) + static_cast<size_t>(norm_group_threads(H)) * norm_groups(H) * 3 * 64;
+}
+constexpr int kNormBwdMaxSmem = 2048 * 4 + kNormBwdThreads * 3 * 64;
 inline int norm_bwd_grid(int rows, int H, int sms) {
   const int groups = norm_groups(H), want = (rows + groups - 1) / groups;
   const int most = sms * (768 / (groups * norm_group_threads(H)));
   return want < most ? (want > 0 ? want : 1) : most;
+}
+
+__device__ __forceinline__ void copy16_async(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))), "l"(gmem)
+               : "memory");
 }
 
 template <typename T, bool RMS, bool BIAS>
@@ -114,7 +126,8 @@ __global__ void __launch_bounds__(kNormBwdThreads, 2) add_norm_bwd_kernel(
     const T* __restrict__ dy, const T* __restrict__ extra, bool extra_is_dy, const T* __restrict__ s,
     const float* __restrict__ w, const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
     float* __restrict__ part, int rows, int H, int NT) {
-  extern __shared__ float sm[];                    // [H]
+  constexpr int N = norm_ring<T>();
+  extern __shared__ __align__(16) float sm[];      // [H], then the ring
   __shared__ float2 red[2][kNormBwdThreads / 32];  // per warp, two rows in turn
   const int groups = blockDim.x / NT, group = threadIdx.x / NT, t = threadIdx.x - group * NT, c = t * 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gw = NT / 32;
@@ -123,30 +136,38 @@ __global__ void __launch_bounds__(kNormBwdThreads, 2) add_norm_bwd_kernel(
   float adw[8], adb[8], abias[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) adw[k] = adb[k] = abias[k] = 0.f;
-  Raw8<T> rv, rd, re, nv, nd, ne;
-  float mu = 0.f, rs = 0.f, nmu = 0.f, nrs = 0.f;
-  auto fetch = [&](int row, Raw8<T>& v, Raw8<T>& d, Raw8<T>& e, float& m, float& q) {
-    const size_t at = static_cast<size_t>(row) * H + c;
-    m = RMS ? 0.f : mean[row];
-    q = rstd[row];
-    if (on) {
-      v.load(s + at);
-      d.load(dy + at);
-      if (extra != nullptr) e.load(extra + at);
+  T* ring = reinterpret_cast<T*>(sm + H);  // [N][3][blockDim.x][8]
+  auto slot = [&](int n, int tensor) { return ring + (static_cast<size_t>(n * 3 + tensor) * blockDim.x + threadIdx.x) * 8; };
+  auto fetch = [&](int row, int n) {
+    if (on && row < rows) {
+      const size_t at = static_cast<size_t>(row) * H + c;
+#pragma unroll
+      for (int h = 0; h < static_cast<int>(sizeof(T)) / 2; ++h) {  // 16 bytes at a time
+        constexpr int V = 16 / sizeof(T);
+        copy16_async(slot(n, 0) + h * V, s + at + h * V);
+        copy16_async(slot(n, 1) + h * V, dy + at + h * V);
+        if (extra != nullptr) copy16_async(slot(n, 2) + h * V, extra + at + h * V);
+      }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   const int step = gridDim.x * groups;
-  int row = blockIdx.x * groups + group, turn = 0;
-  if (row < rows) fetch(row, rv, rd, re, mu, rs);
-  for (; row < rows; row += step, turn ^= 1) {
-    if (row + step < rows) fetch(row + step, nv, nd, ne, nmu, nrs);
-    // unpacked before and again after the barrier: fewer registers stay live across it
+  int row = blockIdx.x * groups + group, turn = 0, n = 0;
+#pragma unroll
+  for (int i = 0; i < N - 1; ++i) fetch(row + i * step, i);
+  float mu = 0.f, rs = 0.f, nmu = 0.f, nrs = 0.f;
+  if (row < rows) mu = RMS ? 0.f : mean[row], rs = rstd[row];
+  for (; row < rows; row += step, turn ^= 1, n = n + 1 == N ? 0 : n + 1) {
+    fetch(row + (N - 1) * step, n == 0 ? N - 1 : n - 1);
+    if (row + step < rows) nmu = RMS ? 0.f : mean[row + step], nrs = rstd[row + step];
+    asm volatile("cp.async.wait_group %0;" ::"n"(N - 1) : "memory");  // this row's copies, which only this thread reads
+    // read before and again after the barrier: fewer registers stay live across it
     auto unpack = [&](float (&v)[8], float (&d)[8], float (&g)[8]) {
-      rv.get(v);
-      rd.get(d);
+      Vec8<T>::load(slot(n, 0), v);
+      Vec8<T>::load(slot(n, 1), d);
       if (extra != nullptr && extra_is_dy) {
         float e[8];
-        re.get(e);
+        Vec8<T>::load(slot(n, 2), e);
 #pragma unroll
         for (int k = 0; k < 8; ++k) d[k] += e[k];
       }
@@ -186,7 +207,7 @@ __global__ void __launch_bounds__(kNormBwdThreads, 2) add_norm_bwd_kernel(
       for (int k = 0; k < 8; ++k) o[k] = rs * (g[k] * d[k] - m1 - v[k] * m2);
       if (extra != nullptr && !extra_is_dy) {
         float r[8];
-        re.get(r);
+        Vec8<T>::load(slot(n, 2), r);
 #pragma unroll
         for (int k = 0; k < 8; ++k) o[k] += r[k];
       }
@@ -196,7 +217,7 @@ __global__ void __launch_bounds__(kNormBwdThreads, 2) add_norm_bwd_kernel(
       }
       Vec8<T>::store(dx + static_cast<size_t>(row) * H + c, o);
     }
-    rv = nv, rd = nd, re = ne, mu = nmu, rs = nrs;
+    mu = nmu, rs = nrs;
   }
   auto combine = [&](float (&acc)[8], int array) {
     for (int q = 0; q < groups; ++q) {

@@ -219,13 +219,14 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> add_norm_bwd(
   at::Tensor part = at::empty({arrays, grid, H}, fopt);
   auto stream = at::cuda::getCurrentCUDAStream();
 #define DQ_BWD(T, RMS, BIAS)                                                                                              \
+  C10_CUDA_CHECK(cudaFuncSetAttribute(add_norm_bwd_kernel<T, RMS, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNormBwdMaxSmem)); \
   add_norm_bwd_kernel<T, RMS, BIAS><<<grid, threads, norm_bwd_smem(H), stream>>>(                                         \
       reinterpret_cast<const T*>(dy.data_ptr()), rows_of<const T>(dy2.has_value() ? dy2 : ds), dy2.has_value(),           \
       reinterpret_cast<const T*>(s.data_ptr()), w.data_ptr<float>(), rms ? nullptr : mean.data_ptr<float>(),              \
       rstd.data_ptr<float>(), reinterpret_cast<T*>(dx.data_ptr()), part.data_ptr<float>(), rows, H, nt)
 #define DQ_BWD_T(T)                                                              \
-  if (rms) { if (want_bias) DQ_BWD(T, true, true); else DQ_BWD(T, true, false); }  \
-  else { if (want_bias) DQ_BWD(T, false, true); else DQ_BWD(T, false, false); }
+  if (rms) { if (want_bias) { DQ_BWD(T, true, true); } else { DQ_BWD(T, true, false); } }  \
+  else { if (want_bias) { DQ_BWD(T, false, true); } else { DQ_BWD(T, false, false); } }
   if (s.scalar_type() == at::kBFloat16) { DQ_BWD_T(__nv_bfloat16) } else { DQ_BWD_T(float) }
 #undef DQ_BWD_T
 #undef DQ_BWD

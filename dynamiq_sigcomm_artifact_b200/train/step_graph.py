@@ -51,7 +51,10 @@ class StepGraph:
         before = counters.snapshot()
         opt.use_hyper = True
         try:
-            with torch.cuda.graph(self.graph, pool=pool, capture_error_mode="thread_local"):
+            # the captured kernels keep their streams' priorities: optimizer steps on the side stream only take SMs that
+            # backward leaves idle
+            with torch.cuda.graph(self.graph, pool=pool, stream=torch.cuda.Stream(tr.device, priority=-1),
+                                  capture_error_mode="thread_local"):
                 self.loss = tr._forward_backward(self.ids, self.labels)
         finally:
             opt.use_hyper = False
