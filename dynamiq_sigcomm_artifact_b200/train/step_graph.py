@@ -12,6 +12,7 @@ trainer then captures the transformer blocks only.
 """
 from __future__ import annotations
 
+import gc
 from typing import Optional
 
 import torch
@@ -50,6 +51,10 @@ class StepGraph:
             self.graph.register_generator_state(gen)
         before = counters.snapshot()
         opt.use_hyper = True
+        # a garbage collection inside the capture could destroy another trainer's graphs, which CUDA does not allow then
+        collecting = gc.isenabled()
+        gc.collect()
+        gc.disable()
         try:
             # the captured kernels keep their streams' priorities: optimizer steps on the side stream only take SMs that
             # backward leaves idle
@@ -58,6 +63,8 @@ class StepGraph:
                 self.loss = tr._forward_backward(self.ids, self.labels)
         finally:
             opt.use_hyper = False
+            if collecting:
+                gc.enable()
             if gen is not None:
                 gen.set_state(rng)
         self.launches = counters.total() - sum(before.values())
