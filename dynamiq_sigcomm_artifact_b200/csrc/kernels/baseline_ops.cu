@@ -15,6 +15,7 @@
 
 #include "../common/exact_div.cuh"
 #include "../common/philox.cuh"
+#include "dependent_launch.cuh"
 
 namespace dq {
 namespace {
@@ -40,6 +41,8 @@ __device__ __forceinline__ float thc_bin(float y, uint32_t byte, float range, co
 __global__ void __launch_bounds__(256) thc_quantize_kernel(float* __restrict__ y, const float* __restrict__ stats, int world,
                                                            float t_over_sqrt_d, int levels, long long d, uint32_t stream,
                                                            uint32_t step, uint32_t seed_lo, uint32_t seed_hi) {
+  wait_for_previous();
+  let_next_start();
   const float range = thc_range(stats, world, t_over_sqrt_d);
   const float top = static_cast<float>(levels - 1);
   const SharedDivisor two_range(__fmul_rn(2.0f, range));
@@ -89,6 +92,8 @@ __global__ void __launch_bounds__(256) thc_quantize_kernel(float* __restrict__ y
 // bin of an odd number of levels gives a zero, which the ordinary division sends down its slow path: see exact_div.cuh.
 __global__ void __launch_bounds__(256) thc_dequantize_kernel(float* __restrict__ total, const float* __restrict__ stats,
                                                              int world, float t_over_sqrt_d, int levels, long long d) {
+  wait_for_previous();
+  let_next_start();
   const float range = thc_range(stats, world, t_over_sqrt_d);
   const float two_range = __fmul_rn(2.0f, range), top = static_cast<float>(levels - 1);
   const float w = static_cast<float>(world), shift = __fmul_rn(w, range);
@@ -125,11 +130,10 @@ void thc_quantize_(at::Tensor y, at::Tensor stats, int64_t world, double t_over_
   if (d == 0) return;
   const int grid = static_cast<int>(std::min<long long>((d + 4095) / 4096, 148 * 8));
   const uint64_t s = static_cast<uint64_t>(seed);
-  thc_quantize_kernel<<<grid, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
-      y.data_ptr<float>(), stats.data_ptr<float>(), static_cast<int>(world), static_cast<float>(t_over_sqrt_d),
+  C10_CUDA_CHECK(launch_dependent(
+      thc_quantize_kernel, grid, 256, 0, at::cuda::getCurrentCUDAStream(), y.data_ptr<float>(), stats.data_ptr<float>(), static_cast<int>(world), static_cast<float>(t_over_sqrt_d),
       static_cast<int>(levels), d, static_cast<uint32_t>(stream), static_cast<uint32_t>(step),
-      static_cast<uint32_t>(s & 0xFFFFFFFFull), static_cast<uint32_t>(s >> 32));
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
+      static_cast<uint32_t>(s & 0xFFFFFFFFull), static_cast<uint32_t>(s >> 32)));
 }
 
 void thc_dequantize_(at::Tensor total, at::Tensor stats, int64_t world, double t_over_sqrt_d, int64_t levels) {
@@ -138,10 +142,9 @@ void thc_dequantize_(at::Tensor total, at::Tensor stats, int64_t world, double t
   const long long d = total.numel();
   if (d == 0) return;
   const int grid = static_cast<int>(std::min<long long>((d + 1023) / 1024, 148 * 8));
-  thc_dequantize_kernel<<<grid, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
-      total.data_ptr<float>(), stats.data_ptr<float>(), static_cast<int>(world), static_cast<float>(t_over_sqrt_d),
-      static_cast<int>(levels), d);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  C10_CUDA_CHECK(launch_dependent(
+      thc_dequantize_kernel, grid, 256, 0, at::cuda::getCurrentCUDAStream(), total.data_ptr<float>(), stats.data_ptr<float>(), static_cast<int>(world), static_cast<float>(t_over_sqrt_d),
+      static_cast<int>(levels), d));
 }
 
 }  // namespace dq

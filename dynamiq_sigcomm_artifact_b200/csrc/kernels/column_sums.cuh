@@ -1,11 +1,11 @@
 // The second half of every column sum: partial rows, one per CTA of the first half, added in a fixed order.
 //
-// The launch is a programmatic dependent one: it is set up while the first half still runs and waits on the device for
-// its end, which takes the launch out of a chain of short kernels (a first half may allow it early with let_next_start();
-// without that, it starts when the first half has ended).  Forked to another stream instead, the sums delayed the GEMMs
-// beside them (26 -> 43 us for a weight gradient of GPT-2 small).
+// A dependent launch (dependent_launch.cuh) behind the first half.  Forked to another stream instead, the sums delayed the
+// GEMMs beside them (26 -> 43 us for a weight gradient of GPT-2 small).
 #pragma once
 #include <cuda_runtime.h>
+
+#include "dependent_launch.cuh"
 
 namespace dq {
 
@@ -14,22 +14,6 @@ inline int device_sms() {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return sms;
-}
-
-// every kernel launched with launch_dependent() calls wait_for_previous() before it touches memory
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename... Params, typename... Args>
-inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                    Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
-  cfg.attrs = attr, cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
 // out[a][c] = sum over the parts of array a: 32 columns x 32 part groups per CTA, blockIdx.y = array

@@ -16,6 +16,7 @@
 #include <torch/extension.h>
 
 #include "../common/rht_codec.cuh"
+#include "dependent_launch.cuh"
 
 namespace dq {
 namespace {
@@ -46,6 +47,8 @@ __global__ void __launch_bounds__(kEdenWarps * 32, 2) eden_compress_kernel(
   __shared__ __align__(16) float sgn[kBlock];
   __shared__ uint32_t sign_words[32];
   __shared__ float cen[L], bnd[L];
+  let_next_start();
+  wait_for_previous();
   for (int i = threadIdx.x; i < L; i += kEdenWarps * 32) {
     cen[i] = levels[i];
     bnd[i] = i < L - 1 ? levels[L + i] : INFINITY;
@@ -120,6 +123,8 @@ __global__ void __launch_bounds__(kEdenWarps * 32, 2) eden_decompress_kernel(
   __shared__ __align__(16) float sgn[kBlock];
   __shared__ uint32_t sign_words[32];
   __shared__ float cen[L];
+  let_next_start();
+  wait_for_previous();
   for (int i = threadIdx.x; i < L; i += kEdenWarps * 32) cen[i] = levels[i];
   eden_signs(sgn, sign_words, 1.0f / 32.0f, step, seed_lo, seed_hi);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -185,9 +190,9 @@ std::tuple<at::Tensor, at::Tensor> eden_compress(at::Tensor x, at::Tensor levels
   const uint64_t s = static_cast<uint64_t>(seed);
   auto stream = at::cuda::getCurrentCUDAStream();
 #define DQ_CALL(B)                                                                                                     \
-  eden_compress_kernel<B><<<eden_grid(nb), kEdenWarps * 32, 0, stream>>>(                                              \
+  C10_CUDA_CHECK(launch_dependent(eden_compress_kernel<B>, eden_grid(nb), kEdenWarps * 32, 0, stream,                                               \
       x.data_ptr<float>(), levels.data_ptr<float>(), reinterpret_cast<uint32_t*>(words.data_ptr<int>()),               \
-      scale.data_ptr<float>(), n, nb, static_cast<uint32_t>(step), static_cast<uint32_t>(s), static_cast<uint32_t>(s >> 32))
+      scale.data_ptr<float>(), n, nb, static_cast<uint32_t>(step), static_cast<uint32_t>(s), static_cast<uint32_t>(s >> 32)))
   DQ_EDEN_SWITCH(DQ_CALL)
 #undef DQ_CALL
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -211,9 +216,9 @@ at::Tensor eden_decompress(at::Tensor words, at::Tensor scale, at::Tensor levels
   const uint64_t s = static_cast<uint64_t>(seed);
   auto stream = at::cuda::getCurrentCUDAStream();
 #define DQ_CALL(B)                                                                                                     \
-  eden_decompress_kernel<B><<<eden_grid(used), kEdenWarps * 32, 0, stream>>>(                                            \
+  C10_CUDA_CHECK(launch_dependent(eden_decompress_kernel<B>, eden_grid(used), kEdenWarps * 32, 0, stream,                                             \
       reinterpret_cast<const uint32_t*>(words.data_ptr<int>()), scale.data_ptr<float>(), levels.data_ptr<float>(),     \
-      out.data_ptr<float>(), n, used, nb, static_cast<uint32_t>(step), static_cast<uint32_t>(s), static_cast<uint32_t>(s >> 32))
+      out.data_ptr<float>(), n, used, nb, static_cast<uint32_t>(step), static_cast<uint32_t>(s), static_cast<uint32_t>(s >> 32)))
   DQ_EDEN_SWITCH(DQ_CALL)
 #undef DQ_CALL
   C10_CUDA_KERNEL_LAUNCH_CHECK();

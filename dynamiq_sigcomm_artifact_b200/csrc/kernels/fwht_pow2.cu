@@ -15,6 +15,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include "dependent_launch.cuh"
+
 namespace dq {
 namespace {
 
@@ -44,6 +46,8 @@ __global__ void __launch_bounds__(kFwhtThreads, 4) fwht_tile_kernel(const float*
                                                                      long long n, int col_log, int first, int lo, int hi,
                                                                      int clean, float scale) {
   __shared__ __align__(16) float sm[kTile];
+  wait_for_previous();
+  let_next_start();
   const int tid = threadIdx.x;
   // tile -> (outer block of 2^(first + rows) values, column group)
   const int row_log = kTileLog - col_log;
@@ -151,15 +155,14 @@ at::Tensor fwht_pow2(at::Tensor x, double scale, bool clean) {
   const unsigned grid = static_cast<unsigned>(std::max<long long>(1, n >> kTileLog));
   const int contiguous = std::min(k, kTileLog);
   float* out = y.data_ptr<float>();
-  fwht_tile_kernel<<<grid, kFwhtThreads, 0, stream>>>(x.data_ptr<float>(), out, n, kTileLog, 0, 0, contiguous, clean ? 1 : 0,
-                                                      k <= kTileLog ? static_cast<float>(scale) : 1.0f);
+  C10_CUDA_CHECK(launch_dependent(fwht_tile_kernel, grid, kFwhtThreads, 0, stream, x.data_ptr<float>(), out, n, kTileLog, 0, 0, contiguous, clean ? 1 : 0,
+                                                      k <= kTileLog ? static_cast<float>(scale) : 1.0f));
   for (int first = kTileLog; first < k;) {
     const int m = std::min(kRowLevels, k - first);
-    fwht_tile_kernel<<<grid, kFwhtThreads, 0, stream>>>(out, out, n, kTileLog - m, first, kTileLog - m, kTileLog, 0,
-                                                        first + m == k ? static_cast<float>(scale) : 1.0f);
+    C10_CUDA_CHECK(launch_dependent(fwht_tile_kernel, grid, kFwhtThreads, 0, stream, out, out, n, kTileLog - m, first, kTileLog - m, kTileLog, 0,
+                                                        first + m == k ? static_cast<float>(scale) : 1.0f));
     first += m;
   }
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
   return y;
 }
 

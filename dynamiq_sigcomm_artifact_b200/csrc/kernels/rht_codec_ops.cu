@@ -17,6 +17,7 @@
 
 #include "../common/rht_codec.cuh"
 #include "../common/tcgen05.cuh"
+#include "dependent_launch.cuh"
 
 namespace dq {
 namespace {
@@ -52,6 +53,8 @@ __global__ void __launch_bounds__(kOpWarps * 32, OP == kOpDecode ? 3 : 2) rht_op
   const float c = OP == kOpDecode ? p.finish_scale : 1.0f;
   for (int e = tid; e < kBlock; e += kOpWarps * 32) sgn[e] = ((sign_words[e >> 5] >> (e & 31)) & 1u) ? -c : c;
   __syncthreads();
+  let_next_start();
+  wait_for_previous();  // the tables above need no memory
 
   T* x = static_cast<T*>(p.x);
   const bool vec_ok = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
@@ -108,8 +111,8 @@ void launch_op(const RhtOpParams& p, int64_t max_warps, cudaStream_t stream) {
   (void)configured;
   // a warp per block, at most the warps the caller grants the operator
   const int64_t want = std::min<int64_t>(p.nblocks, std::max<int64_t>(max_warps, kOpWarps));
-  rht_op_kernel<BITS, T, OP><<<static_cast<unsigned>((want + kOpWarps - 1) / kOpWarps), kOpWarps * 32, kOpSmem, stream>>>(p);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  C10_CUDA_CHECK(launch_dependent(rht_op_kernel<BITS, T, OP>, static_cast<unsigned>((want + kOpWarps - 1) / kOpWarps), kOpWarps * 32,
+                                  kOpSmem, stream, p));
 }
 
 template <typename T, int OP>

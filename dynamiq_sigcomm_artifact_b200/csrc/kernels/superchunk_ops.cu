@@ -9,6 +9,8 @@
 #include <cuda_bf16.h>
 #include <torch/extension.h>
 
+#include "dependent_launch.cuh"
+
 namespace dq {
 namespace {
 
@@ -21,6 +23,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) sc_center_kernel(const T* __restrict__ x, float* __restrict__ resid,
                                                         float* __restrict__ stats, long long n, long long nsc,
                                                         float inv_world) {
+  wait_for_previous();
+  let_next_start();
   const int lane = threadIdx.x & 31;
   const long long warp = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   const long long nwarps = (gridDim.x * static_cast<long long>(blockDim.x)) >> 5;
@@ -57,6 +61,8 @@ __global__ void __launch_bounds__(256) sc_center_kernel(const T* __restrict__ x,
 // copy rate); out is 4-element aligned where this runs, the residual always is
 __global__ void __launch_bounds__(256) sc_add_mean_vec_kernel(const float* __restrict__ resid, const float* __restrict__ mean,
                                                               float* __restrict__ out, long long n4) {
+  wait_for_previous();
+  let_next_start();
   const long long step = gridDim.x * 256ll;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n4; i += 2 * step) {
     const long long j = i + step;
@@ -93,9 +99,9 @@ std::tuple<at::Tensor, at::Tensor> superchunk_center(at::Tensor x, int64_t world
   auto stream = at::cuda::getCurrentCUDAStream();
   const float inv = 1.0f / static_cast<float>(world);
   if (x.scalar_type() == at::kFloat)
-    sc_center_kernel<float><<<grid, 256, 0, stream>>>(x.data_ptr<float>(), resid.data_ptr<float>(), stats.data_ptr<float>(), n, nsc, inv);
+    C10_CUDA_CHECK(launch_dependent(sc_center_kernel<float>, grid, 256, 0, stream, x.data_ptr<float>(), resid.data_ptr<float>(), stats.data_ptr<float>(), n, nsc, inv));
   else
-    sc_center_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), resid.data_ptr<float>(), stats.data_ptr<float>(), n, nsc, inv);
+    C10_CUDA_CHECK(launch_dependent(sc_center_kernel<__nv_bfloat16>, grid, 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), resid.data_ptr<float>(), stats.data_ptr<float>(), n, nsc, inv));
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   return {resid, stats};
 }
@@ -114,9 +120,8 @@ void superchunk_add_mean(at::Tensor resid, at::Tensor mean, at::Tensor out) {
   if (out.scalar_type() == at::kFloat &&
       ((reinterpret_cast<uintptr_t>(out.data_ptr()) | reinterpret_cast<uintptr_t>(resid.data_ptr())) & 15u) == 0 && n >= 4) {
     const long long n4 = n / 4;
-    sc_add_mean_vec_kernel<<<static_cast<int>(std::min<long long>((n4 + 511) / 512, 148LL * 8)), 256, 0, stream>>>(
-        resid.data_ptr<float>(), mean.data_ptr<float>(), out.data_ptr<float>(), n4);
-    C10_CUDA_KERNEL_LAUNCH_CHECK();
+    C10_CUDA_CHECK(launch_dependent(sc_add_mean_vec_kernel, static_cast<unsigned>(std::min<long long>((n4 + 511) / 512, 148LL * 8)), 256, 0,
+                                    stream, resid.data_ptr<float>(), mean.data_ptr<float>(), out.data_ptr<float>(), n4));
     done = 4 * n4;
     if (done == n) return;
   }
