@@ -196,6 +196,7 @@ class Trainer:
         if g is not None and g.addresses != self._graph_addresses():
             self._step_graphs.clear()  # parameters or optimizer state moved: every graph is stale
             g = self._step_graphs[key] = None
+            self._graph_pool = None  # a pool whose graphs are all gone cannot be captured into again
         if g is None:
             if key in self._step_graphs:
                 g = self._capture_step(key, ids, labels)

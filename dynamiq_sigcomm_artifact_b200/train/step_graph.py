@@ -61,6 +61,11 @@ class StepGraph:
             with torch.cuda.graph(self.graph, pool=pool, stream=torch.cuda.Stream(tr.device, priority=-1),
                                   capture_error_mode="thread_local"):
                 self.loss = tr._forward_backward(self.ids, self.labels)
+        except Exception:
+            if gen is not None:  # the registered generator still counts for the capture: eager steps get another one
+                tr._gen = torch.Generator(device=tr.device)
+                tr._gen.set_state(rng)
+            raise
         finally:
             opt.use_hyper = False
             if collecting:
