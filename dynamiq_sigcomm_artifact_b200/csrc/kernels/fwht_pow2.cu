@@ -23,16 +23,33 @@ namespace {
 constexpr int kTileLog = 13, kTile = 1 << kTileLog, kFwhtThreads = 256;
 constexpr int kRowLevels = 10;  // levels of a strided launch: 2^10 rows leave 8 columns
 
+// v[i], v[i + 1] <- sums with v[k], v[k + 1], which become the differences, two values per instruction (the same roundings)
+__device__ __forceinline__ void butterfly2(float (&v)[32], int i, int k) {
+  asm("{\n\t.reg .b64 a, b, m;\n\t"
+      "mov.b64 a, {%0, %1};\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "mov.b64 m, {%4, %4};\n\t"
+      "fma.rn.f32x2 m, b, m, a;\n\t"
+      "add.rn.f32x2 a, a, b;\n\t"
+      "mov.b64 {%0, %1}, a;\n\t"
+      "mov.b64 {%2, %3}, m;\n\t}"
+      : "+f"(v[i]), "+f"(v[i + 1]), "+f"(v[k]), "+f"(v[k + 1])
+      : "f"(-1.0f));
+}
+
 // butterfly on register bit BIT of v, skipped when the level of that bit is not this launch's
 template <int BIT>
 __device__ __forceinline__ void level(float (&v)[32], bool on) {
   if (!on) return;
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
-    if ((i & (1 << BIT)) == 0) {
-      const float a = v[i], b = v[i | (1 << BIT)];
+    if (i & (1 << BIT)) continue;
+    if (BIT == 0) {
+      const float a = v[i], b = v[i | 1];
       v[i] = a + b;
-      v[i | (1 << BIT)] = a - b;
+      v[i | 1] = a - b;
+    } else if ((i & 1) == 0) {
+      butterfly2(v, i, i | (1 << BIT));
     }
   }
 }

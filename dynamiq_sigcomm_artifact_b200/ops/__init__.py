@@ -23,6 +23,8 @@ class NativeLibraryMissing(RuntimeError):
 def load(build_if_missing: bool = False) -> bool:
     """Load ``dq_native.so``; returns True when ``torch.ops.dq`` is usable."""
     global _loaded
+    if _loaded:  # every operator call passes here: no lock once the library is in
+        return True
     with _lock:
         if _loaded:
             return True

@@ -83,7 +83,9 @@ class Eden:
         n = x.numel()
         if x.is_cuda:
             counters.add("eden_compress")
-            flat = x.detach().reshape(-1).float().contiguous()
+            flat = x
+            if x.requires_grad or x.dim() != 1 or x.dtype != torch.float32 or not x.is_contiguous():
+                flat = x.detach().reshape(-1).float().contiguous()
             return (*_ops.require().eden_compress(flat, self._levels_on(x.device), self.bits, self.seed, step), n)
         y = fwht1024(x.reshape(-1).float(), self.seed, step, 0, signs=True, normalize=True)
         pad = (-n) % BLOCK
@@ -100,7 +102,9 @@ class Eden:
         nb = scale.numel()
         if scale.is_cuda:
             counters.add("eden_decompress")
-            return _ops.require().eden_decompress(words.to(scale.device).contiguous(), scale.contiguous(),
+            if words.device != scale.device or not words.is_contiguous():
+                words = words.to(scale.device).contiguous()
+            return _ops.require().eden_decompress(words, scale.contiguous(),
                                                   self._levels_on(scale.device), n, self.bits, self.seed, step)
         bins = unpack_bins(words, self.bits, nb * BLOCK)
         y = self.centroids.to(scale.device)[bins.long()].view(nb, BLOCK) * scale.view(nb, 1)
